@@ -66,7 +66,7 @@ static void free_mg(Hierarchy *h)
   for (auto &g : h->gexec)
     if (g) cudaGraphExecDestroy(g);
   void *ptrs[] = {h->d_cinv, h->d_cpiv, h->d_V, h->d_Z, h->d_w, h->d_ctl, h->d_partial, h->d_x, h->d_b,
-                  h->d_io, h->d_gs_count};
+                  h->d_io};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (h->h_ctl) cudaFreeHost(h->h_ctl);

@@ -157,7 +157,7 @@ struct Hierarchy
   int m = 0;
   double *d_V = nullptr, *d_Z = nullptr, *d_w = nullptr, *d_ctl = nullptr, *d_partial = nullptr;
   double *h_ctl = nullptr; // pinned mirror of the control block
-  int partial_blocks = 0;
+  int gs_stride = 0; // blocks a Gram-Schmidt kernel may have (stride of its partial sums)
   double *d_x = nullptr, *d_b = nullptr; // host-API staging vectors
   // captured multigrid cycle per precision (0 FP64, 1 FP32) and its in/out pointer slot
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
@@ -182,7 +182,6 @@ struct Hierarchy
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int *h_cflag = nullptr;     // pinned copy of the coarse inversion's zero-pivot flag
   bool cflag_pending = false; // copy enqueued, not yet checked
-  unsigned *d_gs_count = nullptr; // arrival counter of the Gram-Schmidt passes' last-block reduction
 };
 
 // ---------------------------------------------------------------------------

@@ -257,154 +257,269 @@ __global__ void coarse_smooth_kernel(int n, int n_active, const int *__restrict_
 // ---------------------------------------------------------------------------
 // dense vector kernels for FGMRES (FP64)
 // ---------------------------------------------------------------------------
-// One fused pass of classical Gram-Schmidt over K basis vectors Y[0..K) (row stride n):
-//   GS_DOTS            partial dots  w . Y_j
-//   GS_AXPY_DOTS_NORM  w -= sum_j coef_j Y_j, then partial dots d_j of the new w with every
-//                      Y_j and ||w||^2; the last block then leaves ||w - sum_j d_j Y_j||^2 =
-//                      ||w||^2 - sum_j d_j^2 (Y orthonormal, d = Y^T w) in *norm_out, so the
-//                      second classical Gram-Schmidt pass needs no third pass: the next basis
-//                      vector (w - Y d) / norm is formed by axpy_scale_kernel
-// Every thread keeps the K basis values of its row in registers; per-block partials go to
-// partial[block * 33 + slot] and are summed in block order by the pass's last block.
-enum { GS_DOTS = 0, GS_AXPY_DOTS_NORM = 1 };
+// Classical Gram-Schmidt twice over K basis vectors Y[0..K) (row stride n) in three kernels
+// that need no reduction kernel, arrival counter or fence between them:
+//   dots       block partials of h1 = Y^T w (gs_dots_kernel, or the row phase of the matrix-free
+//              product, mf64_row_dots_kernel)
+//   axpy-dots  h1 from the partials, w -= Y h1, block partials of h2 = Y^T w and of ||w||^2
+//   axpy-scale h2 and ||w - Y h2||^2 = max(0, ||w||^2 - ||h2||^2) (Y orthonormal) from the
+//              partials, next basis vector (w - Y h2) / norm
+// Every block of a consuming kernel sums all producing blocks' partials itself (at most two
+// blocks per SM produce, so at most 2 * 148 * 32 doubles, read from L2 with every load of a
+// warp in flight) in the same fixed order, so the kernel boundary is the only synchronisation
+// and every block holds the same bits; block 0 stores the coefficients for the host.  Bound by
+// latency (small n) or by L2 reads of the basis (8 K n bytes per pass).  The former last-block
+// reduction (fence, arrival counter, then one block reading the partials slot by slot) cost more
+// than the rows: the axpy-dots pass at K = 20 and 4,225 rows took 11.9 us, now 4 us; the three
+// passes averaged over K = 1..28 at 148,225 rows 5.2, 7.3 and 8.7 us.  Inside a block the K sums
+// of a warp are reduced by exchanging halves (about 32 shuffles for any K) instead of 5 K
+// shuffles.  The minimum of two blocks per SM in the launch bounds is there for the compiler's
+// scheduling: without it the axpy-scale kernel was built with 32 registers, a few loads in
+// flight, and took 12.8 us instead of 8.7.
+constexpr int kGsRowsInFlight = 16; // basis values a thread keeps in flight: rows per thread = 16 / K
 
-// Block partials of NS sums and their reduction by the last block to arrive (an arrival
-// counter, reset by that block): partial[block * 33 + slot], then out[slot] summed in block
-// order (lanes over blocks, then a fixed warp tree).  Every thread of the block calls it.
-// With norm_out, out[0..NS-1) are dot products d_j of a vector with orthonormal vectors and
-// out[NS-1] the vector's squared norm; the last block also stores max(0, out[NS-1] - sum d_j^2).
-template <int NS>
-__device__ __forceinline__ void gs_reduce(const double (&acc)[NS], double *__restrict__ partial,
-                                          double *__restrict__ out, unsigned *__restrict__ counter,
-                                          double *__restrict__ norm_out = nullptr)
+// rows a thread takes at once, so that small K keeps as many loads in flight as large K
+template <int K> constexpr int gs_rows() { return K >= kGsRowsInFlight ? 1 : K >= 8 ? 2 : 4; }
+
+// Sums of N values over a warp: lane l returns the sum of v[l] (l < N), N <= 32.  At each of
+// the five steps a lane passes on the half of its values that the other lane keeps.
+template <int N> __device__ __forceinline__ double warp_sums(double (&v)[N])
 {
-  __shared__ double red[kBlock / 32][NS];
-  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  const int lane = threadIdx.x & 31;
+  int cnt = N;
 #pragma unroll
-  for (int j = 0; j < NS; j++)
+  for (int o = 16; o > 0; o >>= 1)
   {
-    double v = group_sum<32>(acc[j]);
-    if (lane == 0) red[warp][j] = v;
+    const bool hi = lane & o;
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+    {
+      if (j >= o || j >= cnt) continue;
+      if (j + o < cnt)
+      {
+        const double keep = hi ? v[j + o < N ? j + o : j] : v[j], give = hi ? v[j] : v[j + o < N ? j + o : j];
+        v[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+      else
+      {
+        const double other = __shfl_xor_sync(0xffffffffu, v[j], o);
+        v[j] = hi ? 0.0 : v[j] + other;
+      }
+    }
+    cnt = cnt < o ? cnt : o;
+  }
+  return v[0];
+}
+
+// a block's sums of acc[0..N) (and, with NORM, of sq in slot N) into partial[slot * stride +
+// block]; every thread of the block calls it
+template <int N, bool NORM>
+__device__ __forceinline__ void gs_block_sums(double (&acc)[N], double sq, double *__restrict__ partial, int stride)
+{
+  __shared__ double red[kBlock / 32][34];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double t = warp_sums<N>(acc);
+  if (lane < N) red[warp][lane] = t;
+  if (NORM)
+  {
+    sq = group_sum<32>(sq);
+    if (lane == 0) red[warp][N] = sq;
   }
   __syncthreads();
+  constexpr int NS = N + (NORM ? 1 : 0);
   if (threadIdx.x < NS)
   {
-    double t = 0;
-    for (int g = 0; g < kBlock / 32; g++) t += red[g][threadIdx.x];
-    partial[(size_t)blockIdx.x * 33 + threadIdx.x] = t;
-    __threadfence();
-  }
-  __shared__ bool last;
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  // the other blocks' partials are read from L2 (ld.global.cg), eight at a time in flight, and
-  // added in block order
-  for (int j = warp; j < NS; j += kBlock / 32)
-  {
-    double t = 0;
-    for (int b0 = lane; b0 < (int)gridDim.x; b0 += 32 * 8)
-    {
-      double v[8];
+    double s = 0;
 #pragma unroll
-      for (int u = 0; u < 8; u++)
-      {
-        const int b = b0 + 32 * u;
-        v[u] = b < (int)gridDim.x ? __ldcg(partial + (size_t)b * 33 + j) : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < 8; u++) t += v[u];
-    }
-    t = group_sum<32>(t);
-    if (lane == 0) out[j] = t;
+    for (int g = 0; g < kBlock / 32; g++) s += red[g][threadIdx.x];
+    partial[(size_t)threadIdx.x * stride + blockIdx.x] = s;
   }
-  if (norm_out)
-  {
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-      double r = out[NS - 1];
-      for (int j = 0; j < NS - 1; j++) r -= out[j] * out[j];
-      norm_out[0] = r > 0.0 ? r : 0.0;
-    }
-  }
-  if (threadIdx.x == 0) *counter = 0u;
 }
 
-template <int K, int MODE>
-__global__ void __launch_bounds__(kBlock) gs_pass_kernel(int n, const double *__restrict__ Y,
-                                                         double *__restrict__ w,
-                                                         const double *__restrict__ coef,
-                                                         double *__restrict__ partial,
-                                                         double *__restrict__ out, unsigned *__restrict__ counter,
-                                                         double *__restrict__ norm_out)
+// the NS sums over the nb producing blocks into shared memory, in the same order in every
+// block: a warp takes NS / 8 slots at once, its lanes the blocks; ends with a barrier
+template <int NS>
+__device__ __forceinline__ void gs_gather_sums(const double *__restrict__ partial, int stride, int nb,
+                                               double *__restrict__ out)
+{
+  constexpr int W = kBlock / 32, S = (NS + W - 1) / W;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double t[S];
+#pragma unroll
+  for (int s = 0; s < S; s++) t[s] = 0;
+#pragma unroll 4
+  for (int b = lane; b < nb; b += 32)
+#pragma unroll
+    for (int s = 0; s < S; s++)
+      if (warp + s * W < NS) t[s] += __ldcg(partial + (size_t)(warp + s * W) * stride + b);
+  const double r = warp_sums<S>(t);
+  if (lane < S && warp + lane * W < NS) out[warp + lane * W] = r;
+  __syncthreads();
+}
+
+// the basis values of R rows i0, i0 + step, ... (row n - 1 in the place of rows beyond the last):
+// volatile loads, then a point that every value passes, so that no product is scheduled between
+// two loads and all R * K of them are in flight together
+template <int K, int R>
+__device__ __forceinline__ void gs_load_rows(const double *__restrict__ Y, int n, int i0, int step, double (&y)[R][K])
+{
+#pragma unroll
+  for (int q = 0; q < R; q++)
+  {
+    const double *p = Y + min(i0 + q * step, n - 1);
+#pragma unroll
+    for (int j = 0; j < K; j++) asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(y[q][j]) : "l"(p + (size_t)j * n));
+  }
+#pragma unroll
+  for (int q = 0; q < R; q++)
+#pragma unroll
+    for (int j = 0; j < K; j++) asm volatile("" : "+d"(y[q][j]));
+}
+
+// w . Y_j for every j
+template <int K>
+__global__ void __launch_bounds__(kBlock, K <= 24 ? 2 : 1) gs_dots_kernel(int n, const double *__restrict__ Y,
+                                                         const double *__restrict__ w, double *__restrict__ partial,
+                                                         int stride)
 {
   CD_PDL_ENTRY();
-  constexpr int NS = MODE == GS_AXPY_DOTS_NORM ? K + 1 : K;
-  double acc[NS];
+  constexpr int R = gs_rows<K>();
+  double acc[K];
 #pragma unroll
-  for (int j = 0; j < NS; j++) acc[j] = 0;
-  double cf[K];
-#pragma unroll
-  for (int j = 0; j < K; j++) cf[j] = MODE == GS_DOTS ? 0.0 : coef[j];
-  const int stride = gridDim.x * blockDim.x;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+  for (int j = 0; j < K; j++) acc[j] = 0;
+  const int step = gridDim.x * kBlock;
+  for (int i0 = blockIdx.x * kBlock + threadIdx.x; i0 < n; i0 += R * step)
   {
-    double y[K];
+    double wi[R], y[R][K];
 #pragma unroll
-    for (int j = 0; j < K; j++) y[j] = __ldg(Y + (size_t)j * n + i);
-    double wi = w[i];
-    if (MODE != GS_DOTS)
+    for (int q = 0; q < R; q++)
     {
-#pragma unroll
-      for (int j = 0; j < K; j++) wi -= cf[j] * y[j];
-      w[i] = wi;
+      const int i = i0 + q * step;
+      wi[q] = i < n ? w[i] : 0.0;
     }
+    gs_load_rows<K, R>(Y, n, i0, step, y);
 #pragma unroll
-    for (int j = 0; j < K; j++) acc[j] += wi * y[j];
-    if constexpr (MODE == GS_AXPY_DOTS_NORM) acc[NS - 1] += wi * wi;
+    for (int q = 0; q < R; q++)
+#pragma unroll
+      for (int j = 0; j < K; j++) acc[j] += wi[q] * y[q][j];
   }
-  gs_reduce<NS>(acc, partial, out, counter, MODE == GS_AXPY_DOTS_NORM ? norm_out : nullptr);
+  gs_block_sums<K, false>(acc, 0.0, partial, stride);
 }
 
-template <int MODE>
-static void launch_gs(int k, int grid, cudaStream_t st, int n, const double *Y, double *w, const double *coef,
-                      double *partial, double *out, unsigned *counter, double *norm_out = nullptr)
+template <int K>
+__global__ void __launch_bounds__(kBlock, K <= 24 ? 2 : 1) gs_axpy_dots_kernel(int n, const double *__restrict__ Y,
+                                                              double *__restrict__ w, const double *__restrict__ p1,
+                                                              int nb1, double *__restrict__ p2, int stride,
+                                                              double *__restrict__ ctl)
 {
-  switch (k)
+  CD_PDL_ENTRY();
+  __shared__ double h[K];
+  gs_gather_sums<K>(p1, stride, nb1, h);
+  if (blockIdx.x == 0 && threadIdx.x < K) ctl[threadIdx.x] = h[threadIdx.x];
+  constexpr int R = gs_rows<K>();
+  double acc[K], sq = 0;
+#pragma unroll
+  for (int j = 0; j < K; j++) acc[j] = 0;
+  const int step = gridDim.x * kBlock;
+  for (int i0 = blockIdx.x * kBlock + threadIdx.x; i0 < n; i0 += R * step)
   {
-#define CD_GS_CASE(K) case K: (void)cd_launch(gs_pass_kernel<K, MODE>, grid, kBlock, 0, st, n, Y, w, coef, partial, out, counter, norm_out); break;
-    CD_GS_CASE(1) CD_GS_CASE(2) CD_GS_CASE(3) CD_GS_CASE(4) CD_GS_CASE(5) CD_GS_CASE(6) CD_GS_CASE(7)
-    CD_GS_CASE(8) CD_GS_CASE(9) CD_GS_CASE(10) CD_GS_CASE(11) CD_GS_CASE(12) CD_GS_CASE(13) CD_GS_CASE(14)
-    CD_GS_CASE(15) CD_GS_CASE(16) CD_GS_CASE(17) CD_GS_CASE(18) CD_GS_CASE(19) CD_GS_CASE(20) CD_GS_CASE(21)
-    CD_GS_CASE(22) CD_GS_CASE(23) CD_GS_CASE(24) CD_GS_CASE(25) CD_GS_CASE(26) CD_GS_CASE(27) CD_GS_CASE(28)
-    CD_GS_CASE(29) CD_GS_CASE(30) CD_GS_CASE(31) CD_GS_CASE(32)
-#undef CD_GS_CASE
-    default: break;
+    double wi[R], y[R][K];
+#pragma unroll
+    for (int q = 0; q < R; q++)
+    {
+      const int i = i0 + q * step;
+      wi[q] = i < n ? w[i] : 0.0;
+    }
+    gs_load_rows<K, R>(Y, n, i0, step, y);
+#pragma unroll
+    for (int q = 0; q < R; q++)
+    {
+      const int i = i0 + q * step;
+#pragma unroll
+      for (int j = 0; j < K; j++) wi[q] -= h[j] * y[q][j];
+      if (i < n) w[i] = wi[q];
+      else wi[q] = 0.0;
+#pragma unroll
+      for (int j = 0; j < K; j++) acc[j] += wi[q] * y[q][j];
+      sq += wi[q] * wi[q];
+    }
+  }
+  gs_block_sums<K, true>(acc, sq, p2, stride);
+}
+
+// y = (w - sum_j h2_j Y_j) / norm unless the norm is 0, for the next Arnoldi vector; with io,
+// block 0 also sets the cycle graph's (in, out) slot for the next preconditioner application
+template <int K>
+__global__ void __launch_bounds__(kBlock, 2) gs_axpy_scale_kernel(int n, const double *__restrict__ Y,
+                                                               const double *__restrict__ w,
+                                                               const double *__restrict__ p2, int nb2, int stride,
+                                                               double *__restrict__ ctl, double *__restrict__ y_next,
+                                                               double **io, double *z_next)
+{
+  CD_PDL_ENTRY();
+  __shared__ double h[K + 1];
+  gs_gather_sums<K + 1>(p2, stride, nb2, h);
+  double nrm2 = h[K];
+#pragma unroll
+  for (int j = 0; j < K; j++) nrm2 -= h[j] * h[j];
+  nrm2 = nrm2 > 0.0 ? nrm2 : 0.0;
+  if (blockIdx.x == 0)
+  {
+    if (threadIdx.x < K) ctl[33 + threadIdx.x] = h[threadIdx.x];
+    if (threadIdx.x == 0)
+    {
+      ctl[66] = nrm2;
+      if (io)
+      {
+        io[0] = y_next;
+        io[1] = z_next;
+      }
+    }
+  }
+  const double hn = sqrt(nrm2);
+  if (hn == 0) return;
+  const double inv = 1.0 / hn;
+  constexpr int R = gs_rows<K>();
+  const int step = gridDim.x * kBlock;
+  for (int i0 = blockIdx.x * kBlock + threadIdx.x; i0 < n; i0 += R * step)
+  {
+    double wi[R], v[R][K];
+#pragma unroll
+    for (int q = 0; q < R; q++)
+    {
+      const int i = i0 + q * step;
+      wi[q] = i < n ? w[i] : 0.0;
+    }
+    gs_load_rows<K, R>(Y, n, i0, step, v);
+#pragma unroll
+    for (int q = 0; q < R; q++)
+    {
+      const int i = i0 + q * step;
+#pragma unroll
+      for (int j = 0; j < K; j++) wi[q] -= h[j] * v[q][j];
+      if (i < n) y_next[i] = inv * wi[q];
+    }
   }
 }
 
 // Phase 2 of the matrix-free FP64 product fused with the first Gram-Schmidt pass: w = A x from
 // the per-cell products (8-wide incidence records, ascending cell order; Dirichlet rows w = x)
-// and the partial dots w . Y_j of the K basis vectors, reduced like a GS_DOTS pass.
+// and the block partials of w . Y_j.
 template <int K>
-__global__ void __launch_bounds__(kBlock) mf64_row_dots_kernel(int n, int na, const int *__restrict__ inc8,
+__global__ void __launch_bounds__(kBlock, K <= 24 ? 2 : 1) mf64_row_dots_kernel(int n, int na, const int *__restrict__ inc8,
                                                                const double *__restrict__ ybuf,
                                                                const double *__restrict__ x, double *__restrict__ w,
-                                                               const double *__restrict__ Y, double *__restrict__ partial,
-                                                               double *__restrict__ out, unsigned *__restrict__ counter)
+                                                               const double *__restrict__ Y,
+                                                               double *__restrict__ partial, int stride)
 {
   CD_PDL_ENTRY();
   double acc[K];
 #pragma unroll
   for (int j = 0; j < K; j++) acc[j] = 0;
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
+  for (int r = blockIdx.x * kBlock + threadIdx.x; r < n; r += gridDim.x * kBlock)
   {
-    double y[K];
-#pragma unroll
-    for (int j = 0; j < K; j++) y[j] = __ldg(Y + (size_t)j * n + r);
+    double y[1][K];
+    gs_load_rows<K, 1>(Y, n, r, 0, y);
     double s;
     if (r >= na)
       s = x[r];
@@ -422,24 +537,70 @@ __global__ void __launch_bounds__(kBlock) mf64_row_dots_kernel(int n, int na, co
     }
     w[r] = s;
 #pragma unroll
-    for (int j = 0; j < K; j++) acc[j] += s * y[j];
+    for (int j = 0; j < K; j++) acc[j] += s * y[0][j];
   }
-  gs_reduce<K>(acc, partial, out, counter);
+  gs_block_sums<K, false>(acc, 0.0, partial, stride);
 }
 
-static void launch_row_dots(int k, int grid, cudaStream_t st, int n, int na, const int *inc8, const double *ybuf,
-                            const double *x, double *w, const double *Y, double *partial, double *out,
-                            unsigned *counter)
+// blocks of a Gram-Schmidt kernel: two per SM (one where K basis values and sums leave registers
+// for one only), never more than the rows need
+static int gs_grid(const cdgpu_ctx *ctx, int n, int k)
+{
+  const int rows = kBlock * (k >= kGsRowsInFlight ? 1 : k >= 8 ? 2 : 4);
+  return std::max(1, std::min((n + rows - 1) / rows, ctx->sm_count * (k <= 24 ? 2 : 1)));
+}
+
+// blocks of the product's row phase: its gathers want more rows in flight than the plain passes
+static int row_dots_grid(const cdgpu_ctx *ctx, int n)
+{
+  return std::max(1, std::min((n + kBlock - 1) / kBlock, ctx->sm_count * 2));
+}
+
+#define CD_GS_CASES(F)                                                                                    \
+  F(1) F(2) F(3) F(4) F(5) F(6) F(7) F(8) F(9) F(10) F(11) F(12) F(13) F(14) F(15) F(16) F(17) F(18)     \
+  F(19) F(20) F(21) F(22) F(23) F(24) F(25) F(26) F(27) F(28) F(29) F(30) F(31) F(32)
+static void launch_gs_dots(int k, int grid, cudaStream_t st, int n, const double *Y, const double *w, double *partial,
+                           int stride)
 {
   switch (k)
   {
-#define CD_RD_CASE(K) case K: (void)cd_launch(mf64_row_dots_kernel<K>, grid, kBlock, 0, st, n, na, inc8, ybuf, x, w, Y, partial, out, counter); break;
-    CD_RD_CASE(1) CD_RD_CASE(2) CD_RD_CASE(3) CD_RD_CASE(4) CD_RD_CASE(5) CD_RD_CASE(6) CD_RD_CASE(7)
-    CD_RD_CASE(8) CD_RD_CASE(9) CD_RD_CASE(10) CD_RD_CASE(11) CD_RD_CASE(12) CD_RD_CASE(13) CD_RD_CASE(14)
-    CD_RD_CASE(15) CD_RD_CASE(16) CD_RD_CASE(17) CD_RD_CASE(18) CD_RD_CASE(19) CD_RD_CASE(20) CD_RD_CASE(21)
-    CD_RD_CASE(22) CD_RD_CASE(23) CD_RD_CASE(24) CD_RD_CASE(25) CD_RD_CASE(26) CD_RD_CASE(27) CD_RD_CASE(28)
-    CD_RD_CASE(29) CD_RD_CASE(30) CD_RD_CASE(31) CD_RD_CASE(32)
-#undef CD_RD_CASE
+#define CD_GS_CASE(K) case K: (void)cd_launch(gs_dots_kernel<K>, grid, kBlock, 0, st, n, Y, w, partial, stride); break;
+    CD_GS_CASES(CD_GS_CASE)
+#undef CD_GS_CASE
+    default: break;
+  }
+}
+static void launch_gs_axpy_dots(int k, int grid, cudaStream_t st, int n, const double *Y, double *w, const double *p1,
+                                int nb1, double *p2, int stride, double *ctl)
+{
+  switch (k)
+  {
+#define CD_GS_CASE(K) case K: (void)cd_launch(gs_axpy_dots_kernel<K>, grid, kBlock, 0, st, n, Y, w, p1, nb1, p2, stride, ctl); break;
+    CD_GS_CASES(CD_GS_CASE)
+#undef CD_GS_CASE
+    default: break;
+  }
+}
+static void launch_gs_axpy_scale(int k, int grid, cudaStream_t st, int n, const double *Y, const double *w,
+                                 const double *p2, int nb2, int stride, double *ctl, double *y, double **io,
+                                 double *z_next)
+{
+  switch (k)
+  {
+#define CD_GS_CASE(K) case K: (void)cd_launch(gs_axpy_scale_kernel<K>, grid, kBlock, 0, st, n, Y, w, p2, nb2, stride, ctl, y, io, z_next); break;
+    CD_GS_CASES(CD_GS_CASE)
+#undef CD_GS_CASE
+    default: break;
+  }
+}
+static void launch_row_dots(int k, int grid, cudaStream_t st, int n, int na, const int *inc8, const double *ybuf,
+                            const double *x, double *w, const double *Y, double *partial, int stride)
+{
+  switch (k)
+  {
+#define CD_GS_CASE(K) case K: (void)cd_launch(mf64_row_dots_kernel<K>, grid, kBlock, 0, st, n, na, inc8, ybuf, x, w, Y, partial, stride); break;
+    CD_GS_CASES(CD_GS_CASE)
+#undef CD_GS_CASE
     default: break;
   }
 }
@@ -478,49 +639,6 @@ __global__ void scale_norm_kernel(int n, const double *__restrict__ nrm2, const 
     io[1] = z_next;
   }
   if (hn != 0 && i < n) y[i] = (1.0 / hn) * x[i];
-}
-
-// y = (w - sum_j coef_j Y_j) / sqrt(*nrm2) unless *nrm2 == 0: the second Gram-Schmidt pass's
-// update of w (in the order of the GS passes) and the next basis vector in one pass
-template <int K>
-__global__ void __launch_bounds__(256) axpy_scale_kernel(int n, const double *__restrict__ Y,
-                                                         const double *__restrict__ w, const double *__restrict__ coef,
-                                                         const double *__restrict__ nrm2, double *__restrict__ y,
-                                                         double **io, double *z_next)
-{
-  CD_PDL_ENTRY();
-  const double hn = sqrt(*nrm2);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (io && i == 0)
-  {
-    // the cycle graph's (in, out) slot for the next preconditioner application
-    io[0] = y;
-    io[1] = z_next;
-  }
-  if (hn == 0 || i >= n) return;
-  double v[K];
-#pragma unroll
-  for (int j = 0; j < K; j++) v[j] = __ldg(Y + (size_t)j * n + i);
-  double wi = w[i];
-#pragma unroll
-  for (int j = 0; j < K; j++) wi -= coef[j] * v[j];
-  y[i] = (1.0 / hn) * wi;
-}
-
-static void launch_axpy_scale(int k, int grid, cudaStream_t st, int n, const double *Y, const double *w,
-                              const double *coef, const double *nrm2, double *y, double **io, double *z_next)
-{
-  switch (k)
-  {
-#define CD_AS_CASE(K) case K: (void)cd_launch(axpy_scale_kernel<K>, grid, 256, 0, st, n, Y, w, coef, nrm2, y, io, z_next); break;
-    CD_AS_CASE(1) CD_AS_CASE(2) CD_AS_CASE(3) CD_AS_CASE(4) CD_AS_CASE(5) CD_AS_CASE(6) CD_AS_CASE(7)
-    CD_AS_CASE(8) CD_AS_CASE(9) CD_AS_CASE(10) CD_AS_CASE(11) CD_AS_CASE(12) CD_AS_CASE(13) CD_AS_CASE(14)
-    CD_AS_CASE(15) CD_AS_CASE(16) CD_AS_CASE(17) CD_AS_CASE(18) CD_AS_CASE(19) CD_AS_CASE(20) CD_AS_CASE(21)
-    CD_AS_CASE(22) CD_AS_CASE(23) CD_AS_CASE(24) CD_AS_CASE(25) CD_AS_CASE(26) CD_AS_CASE(27) CD_AS_CASE(28)
-    CD_AS_CASE(29) CD_AS_CASE(30) CD_AS_CASE(31) CD_AS_CASE(32)
-#undef CD_AS_CASE
-    default: break;
-  }
 }
 
 __global__ void set_io_kernel(double **io, const double *r, double *z)
@@ -1145,10 +1263,9 @@ int setup_hierarchy_buffers(cdgpu_ctx *ctx, Hierarchy &h, int m)
   }
   if (!h.d_w)
   {
-    h.partial_blocks = std::min(ctx->sm_count * 4, (n + kBlock - 1) / kBlock);
-    if (h.partial_blocks < 1) h.partial_blocks = 1;
+    h.gs_stride = ctx->sm_count * 4; // blocks of a Gram-Schmidt kernel, at most
     if ((rc = dev_alloc(ctx, &h.d_w, n)) || (rc = dev_alloc(ctx, &h.d_ctl, 256)) ||
-        (rc = dev_alloc(ctx, &h.d_partial, (size_t)std::max(h.partial_blocks, ctx->sm_count * 8) * 33)) ||
+        (rc = dev_alloc(ctx, &h.d_partial, (size_t)std::max(2 * 33 * h.gs_stride, ctx->sm_count * 8))) ||
         (rc = dev_alloc(ctx, &h.d_x, n)) || (rc = dev_alloc(ctx, &h.d_b, n)))
       return rc;
     CD_CUDA(ctx, cudaMallocHost((void **)&h.h_ctl, 256 * sizeof(double)));
@@ -1159,8 +1276,6 @@ int setup_hierarchy_buffers(cdgpu_ctx *ctx, Hierarchy &h, int m)
     CD_CUDA(ctx, cudaStreamCreateWithFlags(&h.cstream, cudaStreamNonBlocking));
     CD_CUDA(ctx, cudaMallocHost((void **)&h.h_io, 128 * sizeof(double *)));
     if ((rc = dev_alloc(ctx, &h.d_io, 2))) return rc;
-    if ((rc = dev_alloc(ctx, &h.d_gs_count, 1))) return rc;
-    CD_CUDA(ctx, cudaMemset(h.d_gs_count, 0, sizeof(unsigned)));
   }
   return CDGPU_OK;
 }
@@ -1505,8 +1620,8 @@ static int fgmres(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, co
   CD_CUDA(ctx, cudaMemcpyAsync(h.h_ctl, nrm, sizeof(double), cudaMemcpyDeviceToHost, h.cstream));
   CD_CUDA(ctx, cudaEventRecord(h.ev_beta, h.cstream));
   // Iteration i on the device: the preconditioner on v_i, w = A z_i, the Gram-Schmidt passes,
-  // a copy of the control block to pinned slot i % 2 (on the copy stream, behind an event, so
-  // the iteration does not wait for it) and v_{i+1} = w / ||w||, which needs no host value.
+  // v_{i+1} = w / ||w||, which needs no host value, and a copy of the control block to pinned
+  // slot i % 2 (on the copy stream, behind an event, so the next iteration does not wait for it).
   // The host then applies the Givens rotations and the stopping tests.  While it waits for
   // iteration i it has, as a rule, already enqueued iteration i + 1, so the device does not
   // idle during the host's part; it does not when the residual predicted from the convergence
@@ -1515,37 +1630,37 @@ static int fgmres(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, co
   // arithmetic.
   auto enqueue = [&](int i) -> int {
     int rc2;
-    // the kernel that formed v_i (scale_norm_kernel or axpy_scale_kernel) set the cycle's slot
+    // the kernel that formed v_i (scale_norm_kernel or gs_axpy_scale_kernel) set the cycle's slot
     if ((rc2 = precondition(ctx, h, p, V(i), Z(i), true))) return rc2;
-    int k = i + 1, pb = h.partial_blocks;
-    double *c = ctl_it(i);
+    const int k = i + 1, st = h.gs_stride, grid = gs_grid(ctx, n, k);
+    double *c = ctl_it(i), *p1 = h.d_partial, *p2 = p1 + (size_t)33 * st;
+    int nb1 = grid;
     if (h.mf64 && s.d_inc8)
     {
       // w = A z_i matrix-free, its second phase fused with pass 1: h1 = V^T w
       mf64_cells(ctx, s, Z(i));
       CD_LAUNCHED(ctx);
-      launch_row_dots(k, pb, ctx->stream, n, s.n_active, s.d_inc8, s.d_ybuf64, Z(i), h.d_w, h.d_V, h.d_partial, c,
-                      h.d_gs_count);
+      nb1 = row_dots_grid(ctx, n);
+      launch_row_dots(k, nb1, ctx->stream, n, s.n_active, s.d_inc8, s.d_ybuf64, Z(i), h.d_w, h.d_V, p1, st);
       CD_LAUNCHED(ctx);
     }
     else
     {
       if ((rc2 = finest_spmv(ctx, h, Z(i), h.d_w))) return rc2;
       // pass 1: h1 = V^T w
-      launch_gs<GS_DOTS>(k, pb, ctx->stream, n, h.d_V, h.d_w, nullptr, h.d_partial, c, h.d_gs_count);
+      launch_gs_dots(k, grid, ctx->stream, n, h.d_V, h.d_w, p1, st);
       CD_LAUNCHED(ctx);
     }
     // pass 2: w -= V h1, h2 = V^T w, and ||w - V h2||^2 = ||w||^2 - ||h2||^2
-    launch_gs<GS_AXPY_DOTS_NORM>(k, pb, ctx->stream, n, h.d_V, h.d_w, c, h.d_partial, c + 33, h.d_gs_count,
-                                 c + 66);
+    launch_gs_axpy_dots(k, grid, ctx->stream, n, h.d_V, h.d_w, p1, nb1, p2, st, c);
+    CD_LAUNCHED(ctx);
+    // v_{i+1} = (w - V h2) / ||w - V h2||
+    launch_gs_axpy_scale(k, grid, ctx->stream, n, h.d_V, h.d_w, p2, grid, st, c, V(i + 1), h.d_io, Z(i + 1));
     CD_LAUNCHED(ctx);
     CD_CUDA(ctx, cudaEventRecord(h.ev_ready[i & 1], ctx->stream));
     CD_CUDA(ctx, cudaStreamWaitEvent(h.cstream, h.ev_ready[i & 1], 0));
     CD_CUDA(ctx, cudaMemcpyAsync(h.h_slot + (i & 1) * 80, c, sizeof(double) * 67, cudaMemcpyDeviceToHost, h.cstream));
     CD_CUDA(ctx, cudaEventRecord(h.ev_slot[i & 1], h.cstream));
-    // v_{i+1} = (w - V h2) / ||w - V h2||
-    launch_axpy_scale(k, blocks, ctx->stream, n, h.d_V, h.d_w, c + 33, c + 66, V(i + 1), h.d_io, Z(i + 1));
-    CD_LAUNCHED(ctx);
     return CDGPU_OK;
   };
   // the first restart cycle's v_0 and iteration 0, before ||r0|| is known on the host (if the
@@ -1599,7 +1714,6 @@ static int fgmres(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, co
       CD_CUDA(ctx, cudaEventSynchronize(h.ev_slot[i & 1]));
       const double *c = h.h_slot + (i & 1) * 80;
       const int k = i + 1;
-      // the slot-0 reduction of the last pass holds ||w||^2 (slot 32 of the partials)
       for (int t = 0; t < k; t++) H[(size_t)t * m + i] = c[t] + c[33 + t];
       double hn = std::sqrt(c[66]);
       H[(size_t)(i + 1) * m + i] = hn;
