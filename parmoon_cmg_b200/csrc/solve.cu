@@ -996,6 +996,8 @@ template <typename T> static int cycle(cdgpu_ctx *ctx, Hierarchy &h, CycleState 
   if (cs.p->cycle < 1) cs.rec[i] = 1;
   csr_prolong<T>(ctx, L, s, vc.sol, v.sol, (T)cs.p->gmg_damp);
   CD_LAUNCHED(ctx);
+  // the corrected iterate is not zero, also where no pre-smoothing sweep has cleared the flags
+  cs.sol_zero[i] = cs.active_zero[i] = false;
   return smooth<T>(ctx, h, cs, i, cs.p->post);
 }
 
