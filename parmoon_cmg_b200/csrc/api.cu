@@ -65,7 +65,7 @@ static void free_mg(Hierarchy *h)
   }
   for (auto &g : h->gexec)
     if (g) cudaGraphExecDestroy(g);
-  void *ptrs[] = {h->d_cinv, h->d_cpiv, h->d_V, h->d_Z, h->d_w, h->d_ctl, h->d_partial, h->d_x, h->d_b,
+  void *ptrs[] = {h->d_cinv, h->d_cpiv, h->d_dense, h->d_V, h->d_Z, h->d_w, h->d_ctl, h->d_partial, h->d_x, h->d_b,
                   h->d_io};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -746,8 +746,9 @@ int cdgpu_assemble_hierarchy(cdgpu_ctx *ctx, int mg_id, int disctype, int coarse
   const size_t nl = h->lev.size();
   int rc = CDGPU_OK;
   // The levels are independent: the coarse ones are assembled on the hierarchy's side stream
-  // beside the finest one, and so is the exact coarse inverse once a solve has used it (it
-  // depends on the coarsest level only); the stream of the context waits for both at the end.
+  // beside the finest one, and so are the exact coarse inverse and the dense matrix of the coarse
+  // levels' cycle once a solve has used them (they depend on the coarse levels only); the stream
+  // of the context waits for both streams at the end.
   if (nl > 1)
   {
     if (!h->astream)
@@ -762,6 +763,7 @@ int cdgpu_assemble_hierarchy(cdgpu_ctx *ctx, int mg_id, int disctype, int coarse
     ctx->stream = h->astream;
     for (size_t l = 0; l + 1 < nl && !rc; l++) rc = assemble_space(ctx, *h->lev[l].sp, coarse_disctype, nullptr, false);
     if (!rc && h->d_cinv) rc = refresh_coarse_inverse(ctx, *h);
+    if (!rc && h->dense_level >= 0) rc = refresh_dense_cycle(ctx, *h);
     ctx->stream = main_stream;
     if (rc) return rc;
     CD_CUDA(ctx, cudaEventRecord(h->ev_join, h->astream));

@@ -153,6 +153,14 @@ struct Hierarchy
   double *d_cinv = nullptr; // explicit inverse of the coarsest matrix (exact coarse solve)
   int *d_cpiv = nullptr;    // pivots of its Gauss-Jordan inversion + error flag
   long cinv_version = -1;
+  // the V-cycle of the coarse levels 0..dense_level as one dense matrix (coarse.cuh); the level
+  // the solve's cycles use it from (-1: none), and what the matrix was formed from: the assembly
+  // of every level below and the cycle's parameters
+  int dense_level = -1, dense_built = -1;
+  double *d_dense = nullptr;
+  size_t dense_cap = 0;
+  std::vector<long> dense_versions;
+  cdgpu_solver_params dense_params = {};
   // FGMRES workspace
   int m = 0;
   double *d_V = nullptr, *d_Z = nullptr, *d_w = nullptr, *d_ctl = nullptr, *d_partial = nullptr;
@@ -321,6 +329,9 @@ int apply_fp64_form(cdgpu_ctx *ctx, Space &s, int form, const double *d_x, doubl
 // the explicit inverse of the coarsest level's matrix for the exact coarse solve, when its
 // assembly changed since the last inversion (enqueued on ctx->stream)
 int refresh_coarse_inverse(cdgpu_ctx *ctx, Hierarchy &h);
+// the dense matrix of the coarse levels' V-cycle (coarse.cuh), when an assembly or a parameter
+// changed since it was formed (enqueued on ctx->stream)
+int refresh_dense_cycle(cdgpu_ctx *ctx, Hierarchy &h);
 // the CSR pattern built on the device (pattern.cu)
 int build_pattern_device(cdgpu_ctx *ctx, Space &s, int **d_kcol_out, bool *fallback);
 // tiles of the TMA product for a freshly installed pattern (solve.cu)

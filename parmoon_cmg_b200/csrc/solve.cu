@@ -31,6 +31,7 @@
 #include "csr.cuh"
 #include "mf.cuh"
 #include "mf64.cuh"
+#include "coarse.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -968,6 +969,17 @@ template <typename T> static int coarse_solve(cdgpu_ctx *ctx, Hierarchy &h, Cycl
 
 template <typename T> static int cycle(cdgpu_ctx *ctx, Hierarchy &h, CycleState &cs, int i)
 {
+  if (i == h.dense_level)
+  {
+    // the whole cycle from this level down as one dense product (coarse.cuh)
+    LevelVec<T> &v = vecs<T>(h.lev[i]);
+    const int na = h.lev[i].sp->n_active;
+    (void)cd_launch(dense_cycle_kernel<T>, std::max(1, (na + 7) / 8), 256, 0, ctx->stream, na, (const double *)h.d_dense,
+                    (const T *)v.rhs, v.sol, ctx->pdl_pre ? 1 : 0);
+    CD_LAUNCHED(ctx);
+    cs.sol_zero[i] = cs.active_zero[i] = false;
+    return CDGPU_OK;
+  }
   if (i == 0) return coarse_solve<T>(ctx, h, cs);
   Level &L = h.lev[i], &C = h.lev[i - 1];
   const Space &s = *L.sp, &sc = *C.sp;
@@ -1419,6 +1431,102 @@ int refresh_coarse_inverse(cdgpu_ctx *ctx, Hierarchy &h)
   h.cflag_pending = true;
   h.cinv_version = s.assembly_version;
   return CDGPU_OK;
+}
+
+// The level whose V-cycle a solve with parameters p applies as a dense matrix, or -1.  V-cycles
+// with the exact coarse solve only (the other coarse smoothers iterate until a residual drops and
+// are not linear); below the finest level, whose right-hand side has Dirichlet entries.
+static int choose_dense_level(const Hierarchy &h, const cdgpu_solver_params &p)
+{
+  const int L = (int)h.lev.size();
+  if (p.cycle != 1 || p.coarse_smoother != 17 || p.pre < 0 || p.post < 0) return -1;
+  int best = -1;
+  size_t below = 2 * (size_t)h.lev[0].sp->n_active; // shared memory (doubles) of the levels below
+  for (int l = 1; l <= L - 2 && l < kVMaxLevels; l++)
+  {
+    const size_t na = h.lev[l].sp->n_active;
+    if (na > (size_t)kDenseRows || (below + 3 * na) * sizeof(double) > kVSharedBytes) break;
+    below += 4 * na;
+    best = l;
+  }
+  return best;
+}
+
+int refresh_dense_cycle(cdgpu_ctx *ctx, Hierarchy &h)
+{
+  const int top = h.dense_level;
+  if (top < 1) return CDGPU_OK;
+  const cdgpu_solver_params &p = h.dense_params;
+  std::vector<long> ver;
+  for (int l = 0; l <= top; l++) ver.push_back(h.lev[l].sp->assembly_version);
+  if (h.d_dense && h.dense_built == top && ver == h.dense_versions) return CDGPU_OK;
+  const int na = h.lev[top].sp->n_active;
+  int rc;
+  if ((size_t)na * na > h.dense_cap)
+  {
+    h.dense_cap = 0;
+    if ((rc = dev_alloc(ctx, &h.d_dense, (size_t)na * na))) return rc;
+    h.dense_cap = (size_t)na * na;
+  }
+  VCycleArgs v;
+  v.top = top;
+  v.pre = p.pre;
+  v.post = p.post;
+  v.omega = p.omega;
+  v.damp = p.gmg_damp;
+  v.cinv = h.d_cinv;
+  v.B = h.d_dense;
+  for (int l = 0; l <= top; l++)
+  {
+    const Level &Lv = h.lev[l];
+    const Space &s = *Lv.sp;
+    VLevel &q = v.lev[l];
+    q.na = s.n_active;
+    q.rp = s.d_row_ptr;
+    q.kc = s.d_kcol;
+    q.dirst = s.d_dir_start;
+    q.a = s.d_a;
+    q.diag = s.d_diag;
+    q.prp = Lv.d_p_row;
+    q.pkc = Lv.d_p_col;
+    q.pv = Lv.d_p_val;
+    q.rrp = Lv.d_r_row;
+    q.rkc = Lv.d_r_col;
+    q.rv = Lv.d_r_val;
+    q.row = (int)(s.nnz / std::max(1, s.n_dof));
+    q.prow = (int)(Lv.p_nnz / std::max(1, s.n_dof));
+    q.rrow = l > 0 ? (int)(Lv.p_nnz / std::max(1, h.lev[l - 1].sp->n_dof)) : 1;
+  }
+  // the fewest columns per CTA that leave at most one CTA per SM, as far as shared memory goes
+  int C = 1;
+  while (C < 8 && (na + C - 1) / C > ctx->sm_count && vcycle_layout(v, 2 * C) <= kVSharedBytes) C *= 2;
+  auto kern = C == 1 ? vcycle_matrix_kernel<1> : C == 2 ? vcycle_matrix_kernel<2> : C == 4 ? vcycle_matrix_kernel<4>
+                                                                                           : vcycle_matrix_kernel<8>;
+  const size_t sm = vcycle_layout(v, C);
+  CD_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  (void)cd_launch(kern, std::max(1, (na + C - 1) / C), kVThreads, sm, ctx->stream, v);
+  CD_LAUNCHED(ctx);
+  h.dense_built = top;
+  h.dense_versions = ver;
+  return CDGPU_OK;
+}
+
+// chooses the dense level for a solve, recaptures the cycles when it changed, and forms the matrix
+static int prepare_dense_cycle(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p)
+{
+  const int level = choose_dense_level(h, p);
+  if (level != h.dense_level)
+    for (auto &g : h.gexec)
+      if (g)
+      {
+        cudaGraphExecDestroy(g);
+        g = nullptr;
+      }
+  const cdgpu_solver_params &q = h.dense_params;
+  if (q.pre != p.pre || q.post != p.post || q.omega != p.omega || q.gmg_damp != p.gmg_damp) h.dense_built = -1;
+  h.dense_level = level;
+  h.dense_params = p;
+  return refresh_dense_cycle(ctx, h);
 }
 
 // ---------------------------------------------------------------------------
@@ -1910,6 +2018,7 @@ int run_solve(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, const 
   if (h.mf64 && (rc = ensure_mf64(ctx, fs))) return rc;
   if (!h.mf64 && (rc = tune_tma(ctx, fs))) return rc;
   if (p.coarse_smoother == 17 && (rc = refresh_coarse_inverse(ctx, h))) return rc;
+  if ((rc = prepare_dense_cycle(ctx, h, p))) return rc;
   if (p.precision == 1 && (rc = refresh_mf(ctx, h))) return rc;
   cdgpu_solve_info local{};
   if (!info) info = &local;
@@ -1923,6 +2032,7 @@ int run_solve(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, const 
     if (*h.h_cflag)
     {
       h.cinv_version = -2; // invert again on the next solve
+      h.dense_built = -1;
       return fail(ctx, CDGPU_ERR_INVALID, "exact coarse solve: singular coarse matrix");
     }
   }
