@@ -169,9 +169,10 @@ struct Hierarchy
   double *d_x = nullptr, *d_b = nullptr; // host-API staging vectors
   // captured multigrid cycle per precision (0 FP64, 1 FP32) and its in/out pointer slot
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-  unsigned mf_mask = 0; // levels whose FP32 cycle in gexec[1] uses the matrix-free operator
-  // the running solve applies the finest operator matrix-free in FP64 (mixed form, Q2
-  // hexahedra from the affine constant-coefficient assembly), not from the CSR entries
+  // per precision and level: tensors of the matrix-free operator the captured cycle applies (0: CSR)
+  std::vector<int> mf_tensors[2];
+  // the running solve applies the finest operator matrix-free in FP64 (Q2 hexahedra from the
+  // affine constant-coefficient assembly), not from the CSR entries
   bool mf64 = false;
   cdgpu_solver_params gparams[2] = {};
   long long graph_nodes[2] = {0, 0};

@@ -1,7 +1,7 @@
 // Matrix-free FP64 operator of Q2 hexahedra on affine cells with constant coefficients, by sum
-// factorisation: the product the mixed form's FGMRES iteration applies on the finest level
-// (MatVect / Defect, Blas2.C:11-99, of the matrix TAssembleMat3D assembles) without reading
-// that matrix.
+// factorisation: the product of the FGMRES iteration on the finest level and, in the FP64 form,
+// the defects and Jacobi sweeps of its multigrid cycle (MatVect / Defect, Blas2.C:11-99, and
+// MGLevel3D.C:443, with the matrix TAssembleMat3D assembles) without reading that matrix.
 //
 // The local matrix of a cell is A_c = sum_t coef_{c,t} R_t with the reference tensors R_t of
 // the affine fast path (integrals over [-1,1]^3 of products of the Q2 basis and its
@@ -214,10 +214,10 @@ __global__ void __launch_bounds__(kMf64Warps * 32, 3)
   }
 }
 
-enum { MF64_SPMV = 0, MF64_DEFECT = 1 };
+enum { MF64_SPMV = 0, MF64_DEFECT = 1, MF64_JACOBI = 2 };
 
-// y = sum over a DOF's cells of their contributions (ascending cell order), or d = f - y;
-// Dirichlet rows: y = x, d = f - x.  With partial (defect form), per-block sums of d^2 over
+// y = sum over a DOF's cells of their contributions (ascending cell order), or d = f - y, or the
+// damped Jacobi sweep x + omega (f - y) / diag; Dirichlet rows: y = x, d = f - x, the sweep f.  With partial (defect form), per-block sums of d^2 over
 // all rows, as the CSR defect leaves them.  Grid-stride over rows.
 // With inc8 (the 8-wide incidence records of mf_inc8_kernel) a row reads one record and then
 // its cells' contributions; without, its incidence pointers and entries.
@@ -226,7 +226,8 @@ __global__ void __launch_bounds__(256) mf64_row_kernel(int n, int na, int n_cell
                                                        const int *__restrict__ inc, const int *__restrict__ inc8,
                                                        const double *__restrict__ ybuf,
                                                        const double *__restrict__ x, const double *__restrict__ f,
-                                                       double *__restrict__ out, double *__restrict__ partial)
+                                                       double *__restrict__ out, double *__restrict__ partial,
+                                                       const double *__restrict__ diag, double omega)
 {
   CD_PDL_ENTRY();
   double acc = 0;
@@ -276,6 +277,8 @@ __global__ void __launch_bounds__(256) mf64_row_kernel(int n, int na, int n_cell
       out[r] = d;
       acc += d * d;
     }
+    else if (MODE == MF64_JACOBI)
+      out[r] = r < na ? x[r] + omega * (f[r] - s) / diag[r] : f[r];
     else
       out[r] = s;
   }

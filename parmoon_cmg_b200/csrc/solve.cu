@@ -879,6 +879,85 @@ static void csr_prolong(cdgpu_ctx *ctx, const Level &L, const Space &s, const T 
   launch_csr<T, CM_PROLONG>(ctx, L.p_shape, p, csr_grid(ctx, L.p_shape, p.n_active));
 }
 
+// the matrix-free FP64 operator (mf64.cuh) applies to Q2 hexahedra assembled by the affine
+// constant-coefficient path: the cell coefficients of the last assembly are on the device
+static bool use_mf64(const Space &s)
+{
+  return s.assembled && s.mf_T > 0 && s.d_cellcoef && mf_shape_ok(s.nbf, s.mf_T) && s.dim == 3;
+}
+
+// the 8-wide incidence records of the matrix-free row kernels, built once per space (kept
+// only when every active row has at most 8 cells); synchronises on the first call
+static int ensure_inc8(cdgpu_ctx *ctx, Space &s)
+{
+  if (s.inc8_tried) return CDGPU_OK;
+  s.inc8_tried = true;
+  if (s.n_active <= 0 || (long)s.nbf * s.n_cells >= (long)INT_MAX) return CDGPU_OK;
+  int rc, *flag = nullptr;
+  if ((rc = dev_alloc(ctx, &s.d_inc8, (size_t)s.n_active * 8)) || (rc = dev_alloc(ctx, &flag, 1))) return rc;
+  CD_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(int), ctx->stream));
+  mf_inc8_kernel<<<(s.n_active + 255) / 256, 256, 0, ctx->stream>>>(s.n_active, s.nbf, s.n_cells, s.d_inc_ptr, s.d_inc,
+                                                                   s.d_inc8, flag);
+  CD_LAUNCHED(ctx);
+  int h = 0;
+  CD_CUDA(ctx, cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  CD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  cudaFree(flag);
+  if (h)
+  {
+    cudaFree(s.d_inc8);
+    s.d_inc8 = nullptr;
+  }
+  return CDGPU_OK;
+}
+
+// Levels on which solves apply the operator without the matrix, in both precisions: large enough
+// for the two-kernel form to pay off.  FP64, 32^3 cells: 10.3 us for cells and rows against 39 us
+// for the product and 49 us for the sweep that stream the 190 MB matrix; at 16^3 cells (23 MB, in
+// L2) the CSR kernels take 7 us and stay.
+static bool solve_mf64(const Space &s) { return use_mf64(s) && s.n_cells >= kMfMinCells; }
+
+static int ensure_mf64(cdgpu_ctx *ctx, Space &s)
+{
+  int rc;
+  if (!s.d_ybuf64 && (rc = dev_alloc(ctx, &s.d_ybuf64, (size_t)s.nbf * s.n_cells))) return rc;
+  return ensure_inc8(ctx, s);
+}
+
+// phase 1 of the matrix-free FP64 product: the per-cell products A_c x_c into d_ybuf64
+static void mf64_cells(cdgpu_ctx *ctx, const Space &s, const double *x)
+{
+  static const Mf64Tab tab = mf64_tables();
+  const int groups = (s.n_cells + kMf64Cells - 1) / kMf64Cells;
+  const int grid = std::max(1, std::min(groups, ctx->sm_count * 3));
+  const int cstride = s.mf_T + n_rhs_tensors(s.dim, s.ref_disctype);
+  // the cell data is read before the wait once a launch of this assembly has waited
+  // (inside the captured cycle always: no kernel of the cycle writes it)
+  const int pre = ctx->pdl_pre || s.mf64_safe_version == s.assembly_version ? 1 : 0;
+  if (!pre) s.mf64_safe_version = s.assembly_version;
+  if (s.mf_T == 10)
+    (void)cd_launch(mf64_cell27_kernel<10>, grid, kMf64Warps * 32, 0, ctx->stream, s.n_cells, (const int *)s.d_gn,
+                    (const double *)s.d_cellcoef, cstride, tab, x, s.d_ybuf64, pre);
+  else
+    (void)cd_launch(mf64_cell27_kernel<13>, grid, kMf64Warps * 32, 0, ctx->stream, s.n_cells, (const int *)s.d_gn,
+                    (const double *)s.d_cellcoef, cstride, tab, x, s.d_ybuf64, pre);
+}
+
+// phase 2: y = A x, or d = f - A x with per-block sums of d^2 in partial (grid <= 8 per SM), or a
+// Jacobi sweep
+static int mf64_rows_grid(const cdgpu_ctx *ctx, const Space &s)
+{
+  return std::max(1, std::min((s.n_dof + 255) / 256, ctx->sm_count * 8));
+}
+template <int MODE>
+static void mf64_rows(cdgpu_ctx *ctx, const Space &s, const double *x, const double *f, double *out, double *partial,
+                      const double *diag = nullptr, double omega = 0)
+{
+  (void)cd_launch(mf64_row_kernel<MODE>, mf64_rows_grid(ctx, s), 256, 0, ctx->stream, s.n_dof, s.n_active,
+                  s.n_cells, (const int *)s.d_inc_ptr, (const int *)s.d_inc, (const int *)s.d_inc8,
+                  (const double *)s.d_ybuf64, x, f, out, partial, diag, omega);
+}
+
 template <typename T> static int jacobi_sweep(cdgpu_ctx *ctx, Level &L, T omega)
 {
   LevelVec<T> &v = vecs<T>(L);
@@ -894,6 +973,15 @@ template <typename T> static int jacobi_sweep(cdgpu_ctx *ctx, Level &L, T omega)
       std::swap(v.sol, v.alt);
       return CDGPU_OK;
     }
+  }
+  else if (solve_mf64(s))
+  {
+    mf64_cells(ctx, s, v.sol);
+    CD_LAUNCHED(ctx);
+    mf64_rows<MF64_JACOBI>(ctx, s, v.sol, v.rhs, v.alt, nullptr, s.d_diag, omega);
+    CD_LAUNCHED(ctx);
+    std::swap(v.sol, v.alt);
+    return CDGPU_OK;
   }
   csr_jacobi<T>(ctx, s, v.sol, v.rhs, v.alt, omega);
   CD_LAUNCHED(ctx);
@@ -997,6 +1085,13 @@ template <typename T> static int cycle(cdgpu_ctx *ctx, Hierarchy &h, CycleState 
       mf_rows<MF_DEFECT>(ctx, s, v.sol, v.rhs, s.d_diag32, v.def, 0.f);
       done = true;
     }
+  }
+  else if (solve_mf64(s))
+  {
+    mf64_cells(ctx, s, v.sol);
+    CD_LAUNCHED(ctx);
+    mf64_rows<MF64_DEFECT>(ctx, s, v.sol, v.rhs, v.def, nullptr);
+    done = true;
   }
   if (!done) csr_defect<T>(ctx, s, v.sol, v.rhs, v.def, nullptr, defect_grid<T>(ctx, s));
   CD_LAUNCHED(ctx);
@@ -1539,76 +1634,6 @@ int spmv64(cdgpu_ctx *ctx, const Space &s, const double *x, double *y)
   return CDGPU_OK;
 }
 
-// the matrix-free FP64 operator (mf64.cuh) applies to Q2 hexahedra assembled by the affine
-// constant-coefficient path: the cell coefficients of the last assembly are on the device
-static bool use_mf64(const Space &s)
-{
-  return s.assembled && s.mf_T > 0 && s.d_cellcoef && mf_shape_ok(s.nbf, s.mf_T) && s.dim == 3;
-}
-
-// the 8-wide incidence records of the matrix-free row kernels, built once per space (kept
-// only when every active row has at most 8 cells); synchronises on the first call
-static int ensure_inc8(cdgpu_ctx *ctx, Space &s)
-{
-  if (s.inc8_tried) return CDGPU_OK;
-  s.inc8_tried = true;
-  if (s.n_active <= 0 || (long)s.nbf * s.n_cells >= (long)INT_MAX) return CDGPU_OK;
-  int rc, *flag = nullptr;
-  if ((rc = dev_alloc(ctx, &s.d_inc8, (size_t)s.n_active * 8)) || (rc = dev_alloc(ctx, &flag, 1))) return rc;
-  CD_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(int), ctx->stream));
-  mf_inc8_kernel<<<(s.n_active + 255) / 256, 256, 0, ctx->stream>>>(s.n_active, s.nbf, s.n_cells, s.d_inc_ptr, s.d_inc,
-                                                                   s.d_inc8, flag);
-  CD_LAUNCHED(ctx);
-  int h = 0;
-  CD_CUDA(ctx, cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  CD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  cudaFree(flag);
-  if (h)
-  {
-    cudaFree(s.d_inc8);
-    s.d_inc8 = nullptr;
-  }
-  return CDGPU_OK;
-}
-
-static int ensure_mf64(cdgpu_ctx *ctx, Space &s)
-{
-  int rc;
-  if (!s.d_ybuf64 && (rc = dev_alloc(ctx, &s.d_ybuf64, (size_t)s.nbf * s.n_cells))) return rc;
-  return ensure_inc8(ctx, s);
-}
-
-// phase 1 of the matrix-free FP64 product: the per-cell products A_c x_c into d_ybuf64
-static void mf64_cells(cdgpu_ctx *ctx, const Space &s, const double *x)
-{
-  static const Mf64Tab tab = mf64_tables();
-  const int groups = (s.n_cells + kMf64Cells - 1) / kMf64Cells;
-  const int grid = std::max(1, std::min(groups, ctx->sm_count * 3));
-  const int cstride = s.mf_T + n_rhs_tensors(s.dim, s.ref_disctype);
-  // the cell data is read before the wait once a launch of this assembly has waited
-  const int pre = s.mf64_safe_version == s.assembly_version ? 1 : 0;
-  if (!pre) s.mf64_safe_version = s.assembly_version;
-  if (s.mf_T == 10)
-    (void)cd_launch(mf64_cell27_kernel<10>, grid, kMf64Warps * 32, 0, ctx->stream, s.n_cells, (const int *)s.d_gn,
-                    (const double *)s.d_cellcoef, cstride, tab, x, s.d_ybuf64, pre);
-  else
-    (void)cd_launch(mf64_cell27_kernel<13>, grid, kMf64Warps * 32, 0, ctx->stream, s.n_cells, (const int *)s.d_gn,
-                    (const double *)s.d_cellcoef, cstride, tab, x, s.d_ybuf64, pre);
-}
-
-// phase 2: y = A x, or d = f - A x with per-block sums of d^2 in partial (grid <= 8 per SM)
-static int mf64_rows_grid(const cdgpu_ctx *ctx, const Space &s)
-{
-  return std::max(1, std::min((s.n_dof + 255) / 256, ctx->sm_count * 8));
-}
-template <int MODE>
-static void mf64_rows(cdgpu_ctx *ctx, const Space &s, const double *x, const double *f, double *out, double *partial)
-{
-  (void)cd_launch(mf64_row_kernel<MODE>, mf64_rows_grid(ctx, s), 256, 0, ctx->stream, s.n_dof, s.n_active,
-                  s.n_cells, (const int *)s.d_inc_ptr, (const int *)s.d_inc, (const int *)s.d_inc8,
-                  (const double *)s.d_ybuf64, x, f, out, partial);
-}
-
 // y = A x on the finest level: matrix-free in FP64 where the solve chose it, else the CSR entries
 static int finest_spmv(cdgpu_ctx *ctx, Hierarchy &h, const double *x, double *y)
 {
@@ -1975,25 +2000,28 @@ static int prepare_mf(cdgpu_ctx *ctx, Space &s)
   return CDGPU_OK;
 }
 
-// FP32 copies for the matrix-free operator of every level that has one; the captured FP32
-// cycle is recaptured when the set of such levels changes
-static int refresh_mf(cdgpu_ctx *ctx, Hierarchy &h)
+// What the matrix-free levels of a solve need: FP32 copies for the mixed form's cycle, per-cell
+// buffers for the FP64 products.  The captured cycle is recaptured when the set of such levels or
+// their number of tensors (the kernels' template argument) changes.
+static int refresh_mf(cdgpu_ctx *ctx, Hierarchy &h, int precision)
 {
-  unsigned mask = 0;
+  std::vector<int> tensors(h.lev.size(), 0);
+  int rc;
   for (size_t l = 0; l < h.lev.size(); l++)
   {
     Space &s = *h.lev[l].sp;
+    const bool finest = l + 1 == h.lev.size();
+    if (solve_mf64(s) && (finest || precision == 0) && (rc = ensure_mf64(ctx, s))) return rc;
     if (s.mf_T <= 0 || s.n_cells < kMfMinCells || !mf_shape_ok(s.nbf, s.mf_T)) continue;
-    int rc = prepare_mf(ctx, s);
-    if (rc) return rc;
-    mask |= 1u << l;
+    if (precision == 1 && (rc = prepare_mf(ctx, s))) return rc;
+    if (precision == 1 || solve_mf64(s)) tensors[l] = s.mf_T;
   }
-  if (mask != h.mf_mask && h.gexec[1])
+  if (tensors != h.mf_tensors[precision] && h.gexec[precision])
   {
-    cudaGraphExecDestroy(h.gexec[1]);
-    h.gexec[1] = nullptr;
+    cudaGraphExecDestroy(h.gexec[precision]);
+    h.gexec[precision] = nullptr;
   }
-  h.mf_mask = mask;
+  h.mf_tensors[precision] = tensors;
   return CDGPU_OK;
 }
 
@@ -2010,16 +2038,15 @@ int run_solve(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, const 
   if (p.coarse_smoother != 17 && h.lev[0].sp->n_dof > 6000)
     return fail(ctx, CDGPU_ERR_UNSUPPORTED, "solve: coarse smoother loop needs a coarsest level below 6000 DOFs");
   int rc;
-  // the mixed form applies the finest operator of its FGMRES iteration matrix-free in FP64 on
-  // levels large enough for the per-cell form to pay off; the FP64 form keeps the CSR entries,
-  // whose bulk-copy kernels are tuned once per pattern, before any capture
+  // both forms apply the finest operator matrix-free in FP64 on levels large enough for the
+  // per-cell form to pay off; the FP64 form's CSR product, which other callers apply, is tuned
+  // once per pattern, before any capture
   Space &fs = *h.lev.back().sp;
-  h.mf64 = p.precision == 1 && use_mf64(fs) && fs.n_cells >= kMfMinCells;
-  if (h.mf64 && (rc = ensure_mf64(ctx, fs))) return rc;
-  if (!h.mf64 && (rc = tune_tma(ctx, fs))) return rc;
+  h.mf64 = solve_mf64(fs);
+  if (p.precision == 0 && (rc = tune_tma(ctx, fs))) return rc;
   if (p.coarse_smoother == 17 && (rc = refresh_coarse_inverse(ctx, h))) return rc;
   if ((rc = prepare_dense_cycle(ctx, h, p))) return rc;
-  if (p.precision == 1 && (rc = refresh_mf(ctx, h))) return rc;
+  if ((rc = refresh_mf(ctx, h, p.precision))) return rc;
   cdgpu_solve_info local{};
   if (!info) info = &local;
   if (p.solver == 11) rc = fixed_point(ctx, h, p, d_rhs, d_sol, info);

@@ -19,7 +19,7 @@ import scipy.sparse as sps
 import scipy.sparse.linalg as spl
 
 from parmoon_cmg_b200 import mesh
-from parmoon_cmg_b200.system import SUPG, Context, coeffs, solver_params
+from parmoon_cmg_b200.system import GALERKIN, SUPG, Context, coeffs, solver_params
 
 pytestmark = pytest.mark.gpu
 
@@ -33,7 +33,7 @@ def ctx():
     c.close()
 
 
-def hierarchy(ctx, oracle_lib, dim, order, n0, L):
+def hierarchy(ctx, oracle_lib, dim, order, n0, L, disc=SUPG):
     co = coeffs(0, eps=1e-2, b=(0.8, 0.6) if dim == 2 else (0.6, 0.64, 0.48), c=0.3, f=1.0)
     spaces, parents = mesh.structured_hierarchy(dim, order, n0, L)
     levels, sids = [], []
@@ -41,7 +41,7 @@ def hierarchy(ctx, oracle_lib, dim, order, n0, L):
         sid = ctx.upload_space(sp)
         nnz = ctx.build_pattern(sid)
         ctx.set_coeffs(sid, co)
-        ent, _ = ctx.assemble(sid, SUPG, sp["n_dof"], nnz)
+        ent, _ = ctx.assemble(sid, disc, sp["n_dof"], nnz)
         rp, kc = ctx.get_pattern(sid, sp["n_dof"], nnz)
         lv = dict(A=sps.csr_matrix((ent, kc, rp), shape=(sp["n_dof"],) * 2), na=sp["n_active"])
         lv["d"] = lv["A"].diagonal()
@@ -110,6 +110,26 @@ def test_one_cycle(ctx, oracle_lib, dim, order, n0, L, pre, post, omega, damp, w
         x, info = ctx.solve(mg, prm, f, np.zeros(n))
         err = np.abs(x - ref).max() / np.abs(ref).max()
         print(f"precision {precision}: {err:.2e}")
+        assert err <= tol
+
+
+@pytest.mark.parametrize("disc", [GALERKIN, SUPG])
+def test_one_cycle_with_matrix_free_sweeps(ctx, oracle_lib, disc):
+    """32^3 Q2 cells: the finest level's sweeps and defect are applied without the matrix in both
+    forms (10 and 13 tensors), the coarse levels as above.  The mixed form's tensor-core products
+    round their inputs to TF32 (2^-11 relative), 5e-3."""
+    sids, parents, levels = hierarchy(ctx, oracle_lib, 3, 2, 2, 5, disc)
+    mg = ctx.hierarchy(sids, parents)
+    n, na = levels[-1]["A"].shape[0], levels[-1]["na"]
+    f = np.random.default_rng(disc).standard_normal(n)
+    start = f.copy()
+    start[:na] = 0.0
+    ref = cycle(levels, 4, f, start, 2, 2, 0.8, 1.0, 1)
+    for precision, tol in ((0, 1e-11), (1, 5e-3)):
+        prm = solver_params(solver=11, precision=precision, maxit=1, red_factor=0.0, div_factor=1e30)
+        x, info = ctx.solve(mg, prm, f, np.zeros(n))
+        err = np.abs(x - ref).max() / np.abs(ref).max()
+        print(f"disc {disc} precision {precision}: {err:.2e}")
         assert err <= tol
 
 
