@@ -25,6 +25,13 @@ struct RefElement
   std::vector<double> phi, dphi, hphi; // nq x nbf, nq x nbf x dim, nq x nbf x dim x dim
 };
 void make_ref_element(int dim, int order, RefElement &re);
+// one-dimensional tables in the order of the rule's points (3 for order 1, 4 for order 2): points,
+// weights, values, derivatives and second derivatives of the Lagrange basis
+struct QuadTab
+{
+  double x[4], w[4], B[4][3], G[4][3], H[4][3];
+};
+void make_quad_tab(int order, QuadTab &t);
 void basis_eval(int dim, int order, const double *xi, double *val, double *grad);
 int n_tensors(int dim, int disctype);
 int n_rhs_tensors(int dim, int disctype);

@@ -123,6 +123,14 @@ void make_ref_element(int dim, int order, RefElement &re)
                &re.hphi[q * re.nbf * dim * dim]);
 }
 
+void make_quad_tab(int order, QuadTab &t)
+{
+  t = QuadTab{};
+  const int n1 = order == 1 ? 3 : 4;
+  gauss1d(n1, t.x, t.w);
+  for (int q = 0; q < n1; q++) lag1d(order, t.x[q], t.B[q], t.G[q], t.H[q]);
+}
+
 // ---------------------------------------------------------------------------
 // Reference tensors of the affine fast path.  On a parallelogram/parallelepiped with
 // constant coefficients every term of the local forms (src/FE/ConvDiff2D.C:32-162,
