@@ -55,6 +55,11 @@ struct BLevel
   const int *rrp = nullptr, *rkc = nullptr; // R = P^T: rows of the coarser level
   const float *rv = nullptr;
   const double *cinv = nullptr; // coarsest depth: inverse of the active block
+  // colour classes: class q is color_rows[color_ptr[q] .. color_ptr[q + 1])
+  const int *color_ptr = nullptr;
+  int n_colors = 0;
+  // depth 0: the first depth of the levels one block takes (b_cta_cycle), and the level count
+  int cta_top = 0, levels = 0;
 };
 
 // FGMRES control block of one instance
@@ -86,6 +91,8 @@ struct BInst
   bool used = false;
   int mg = -1, L = 0, state = ST_EMPTY;
   bool reported = false, tcd = false;
+  int cta_top = 0;       // see BLevel
+  size_t cta_smem = 0;   // shared memory of its block in b_cta_cycle
   size_t bytes = 0;
   std::vector<void *> allocs;
   // one allocation per instance, carved by balloc into its arrays (256-byte aligned); arrays
@@ -124,6 +131,7 @@ struct Batch
   int *d_loop = nullptr;        // iterations left in the current call
   int loop_mode = -1;           // -1 not tried, 0 host loop, 1 graph with PDL, 2 graph without
   long long loop_launches = 0, host_iterations = 0;
+  size_t cta_smem = 0; // shared memory of b_cta_cycle for the running set
   std::vector<BTab> smooth, restrict_, coarse;
   std::vector<std::vector<BTab>> color;
   std::vector<int> ncolor_max;
@@ -222,10 +230,10 @@ __global__ void b_mg_start(BTab t, const BCtl *__restrict__ ctl, const BLevel *_
   }
 }
 
-// damped Jacobi sweep v[1-src] = v[src] + omega D^{-1} (f - A v[src]); first = active part
-// of v[src] is zero, so only Dirichlet columns (from dirst) contribute
-__global__ void b_jacobi(BTab t, const BCtl *__restrict__ ctl, const BLevel *__restrict__ lev, int depth, int src,
-                         int first, float omega)
+// First damped Jacobi sweep of depth `depth` when the active part of v[src] is zero: only Dirichlet
+// columns (from dirst) contribute
+__global__ void b_jacobi_first(BTab t, const BCtl *__restrict__ ctl, const BLevel *__restrict__ lev, int depth, int src,
+                               float omega)
 {
   CD_PDL_ENTRY();
   const int lane = threadIdx.x % 4;
@@ -235,103 +243,141 @@ __global__ void b_jacobi(BTab t, const BCtl *__restrict__ ctl, const BLevel *__r
     if (!stepping(ctl[slot])) continue;
     const BLevel &L = lev[slot * kMaxDepth + depth];
     const int r = (vb - t.bstart[k]) * kCsrRows + threadIdx.x / 4;
-    const bool valid = r < L.n;
+    if (r >= L.n || lane != 0) continue;
     const float *x = L.v[src];
-    float *y = L.v[1 - src];
-    if (first)
+    if (r >= L.na)
+      L.v[1 - src][r] = L.rhs[r];
+    else
     {
-      if (valid && lane == 0)
+      float s = L.rhs[r];
+      for (int j = L.dirst[r]; j < L.rp[r + 1]; j++) s -= L.a32[j] * x[L.kc[j]];
+      L.v[1 - src][r] = omega * s / L.d32[r];
+    }
+  }
+}
+
+// The grouped row operations of the cycle, y_r = epilogue((A x)_r) with 4 threads per row:
+//   BR_JACOBI    v[dst] = v[src] + omega D^{-1} (f - A v[src]), Dirichlet rows f
+//   BR_COLOR     one colour class of an SOR sweep, in place on v[0]
+//   BR_DEFECT    def = f - A v[src]
+//   BR_RESTRICT  coarse f = R def on active coarse rows (zero elsewhere), coarse v[0] = 0
+//   BR_PROLONG   v[dst] += omega P (coarse v[src]) on active rows
+// A block takes a contiguous range of virtual blocks, so it looks an instance up once and then
+// walks its rows, the next rows' pointers and entries loaded while the present ones are summed;
+// what the first rows need of tables and matrices (written by no kernel of an iteration) is read
+// before the wait for the predecessor, and the successor is let in at once to do the same.  The
+// launches of a batch are chains of dependent loads (table, level, row list, row pointers,
+// entries, x): with a block per 64 rows, all of them behind the wait, a colour class of a few
+// thousand rows took 3.5-4.2 us and a sweep over 16 x 66,049 rows 84 us.
+enum { BR_JACOBI = 0, BR_COLOR = 1, BR_DEFECT = 2, BR_RESTRICT = 3, BR_PROLONG = 4 };
+
+struct BRowArgs
+{
+  BTab t;
+  const BCtl *ctl;
+  const BLevel *lev;
+  int depth, src, dst;
+  float omega;
+  const int *cstart; // colour class: first position of item k in its level's row list, K + k: count
+};
+
+// the item of virtual block vb, by a whole warp: 32 bounds at a time
+__device__ __forceinline__ int find_item_warp(const BTab &t, int vb)
+{
+  const int lane = threadIdx.x & 31;
+  int lo = 0, n = t.K;
+  while (n > 1)
+  {
+    const int step = (n + 31) >> 5, i = lo + lane * step;
+    const unsigned m = __ballot_sync(0xffffffffu, i < lo + n && __ldg(t.bstart + i) <= vb);
+    const int c = __popc(m) - 1;
+    n = min(step, n - c * step);
+    lo += c * step;
+  }
+  return lo;
+}
+
+// Blocks per SM (40 stationary instances with SSOR and 16 time-dependent ones with Jacobi, solve
+// phases included: 62.5 and 32.2 ms with 4, 66.9 and 31.7 with 5, 73.5 and 36.2 with 6, whose
+// registers leave fewer loads in flight).
+constexpr int kRowBlocks = 4;
+template <int OP> __global__ void __launch_bounds__(kNT, kRowBlocks) b_rows(const __grid_constant__ BRowArgs p)
+{
+  CD_PDL_TRIGGER();
+  constexpr int U = 8;
+  const int lane = threadIdx.x & 3, sub = threadIdx.x >> 2;
+  const int v1 = (int)((long)p.t.total * (blockIdx.x + 1) / gridDim.x);
+  int vb = (int)((long)p.t.total * blockIdx.x / gridDim.x);
+  int k = find_item_warp(p.t, vb);
+  bool waited = false;
+  while (vb < v1)
+  {
+    const int slot = __ldg(p.t.item + k), b0 = __ldg(p.t.bstart + k), ve = min(v1, __ldg(p.t.bstart + k + 1));
+    const BLevel &L = p.lev[slot * kMaxDepth + p.depth], &C = p.lev[slot * kMaxDepth + p.depth + 1];
+    const int *rp = OP == BR_RESTRICT ? L.rrp : OP == BR_PROLONG ? L.prp : L.rp;
+    const int *kc = OP == BR_RESTRICT ? L.rkc : OP == BR_PROLONG ? L.pkc : L.kc;
+    const float *a = OP == BR_RESTRICT ? L.rv : OP == BR_PROLONG ? L.pv : L.a32;
+    const float *x = OP == BR_RESTRICT ? L.def : OP == BR_PROLONG ? C.v[p.src] : OP == BR_COLOR ? L.v[0] : L.v[p.src];
+    const int n = OP == BR_RESTRICT ? L.nc : OP == BR_PROLONG ? L.na : OP == BR_COLOR ? __ldg(p.cstart + p.t.K + k) : L.n;
+    const int na = OP == BR_RESTRICT ? L.nca : OP == BR_JACOBI ? L.na : n; // rows with a sum
+    const int *list = OP == BR_COLOR ? L.color_rows + __ldg(p.cstart + k) : nullptr;
+    const int i1 = min(n, (ve - b0) * kCsrRows);
+    int i = (vb - b0) * kCsrRows + sub, r = 0, b = 0, e = 0, c[U];
+    float v[U];
+    auto fetch = [&]() {
+      r = OP == BR_COLOR ? (i < i1 ? __ldg(list + i) : 0) : i;
+      b = e = 0;
+      if (i < i1 && (OP == BR_COLOR || i < na))
       {
-        if (r >= L.na) y[r] = L.rhs[r];
-        else
-        {
-          float s = L.rhs[r];
-          for (int j = L.dirst[r]; j < L.rp[r + 1]; j++) s -= L.a32[j] * x[L.kc[j]];
-          y[r] = omega * s / L.d32[r];
-        }
+        b = __ldg(rp + r);
+        e = __ldg(rp + r + 1);
       }
-      continue;
-    }
-    const float s = row4<float, float>(L.rp, L.kc, L.a32, x, r, valid && r < L.na, lane);
-    if (valid && lane == 0) y[r] = r < L.na ? x[r] + omega * (L.rhs[r] - s) / L.d32[r] : L.rhs[r];
-  }
-}
-
-// one colour class of an SOR sweep, in place on v[0]
-__global__ void b_color(BTab t, const BCtl *__restrict__ ctl, const BLevel *__restrict__ lev, int depth,
-                        const int *__restrict__ cstart, float omega)
-{
-  CD_PDL_ENTRY();
-  const int lane = threadIdx.x % 4;
-  for (int vb = blockIdx.x; vb < t.total; vb += gridDim.x)
-  {
-    const int k = find_item(t, vb), slot = t.item[k];
-    if (!stepping(ctl[slot])) continue;
-    const BLevel &L = lev[slot * kMaxDepth + depth];
-    // cstart[k]: first position of this colour in L.color_rows, cstart[K + k]: count
-    const int i = (vb - t.bstart[k]) * kCsrRows + threadIdx.x / 4;
-    const bool valid = i < cstart[t.K + k];
-    const int r = valid ? L.color_rows[cstart[k] + i] : 0;
-    float *x = L.v[0];
-    const float s = row4<float, float>(L.rp, L.kc, L.a32, x, r, valid, lane);
-    if (valid && lane == 0) x[r] += omega * (L.rhs[r] - s) / L.d32[r];
-  }
-}
-
-// def = f - A v[src]
-__global__ void b_defect(BTab t, const BCtl *__restrict__ ctl, const BLevel *__restrict__ lev, int depth, int src)
-{
-  CD_PDL_ENTRY();
-  const int lane = threadIdx.x % 4;
-  for (int vb = blockIdx.x; vb < t.total; vb += gridDim.x)
-  {
-    const int k = find_item(t, vb), slot = t.item[k];
-    if (!stepping(ctl[slot])) continue;
-    const BLevel &L = lev[slot * kMaxDepth + depth];
-    const int r = (vb - t.bstart[k]) * kCsrRows + threadIdx.x / 4;
-    const bool valid = r < L.n;
-    const float s = row4<float, float>(L.rp, L.kc, L.a32, L.v[src], r, valid, lane);
-    if (valid && lane == 0) L.def[r] = L.rhs[r] - s;
-  }
-}
-
-// coarse rhs = R def on active coarse rows (zero elsewhere), coarse v[0] = 0
-__global__ void b_restrict(BTab t, const BCtl *__restrict__ ctl, const BLevel *__restrict__ lev, int depth)
-{
-  CD_PDL_ENTRY();
-  const int lane = threadIdx.x % 4;
-  for (int vb = blockIdx.x; vb < t.total; vb += gridDim.x)
-  {
-    const int k = find_item(t, vb), slot = t.item[k];
-    if (!stepping(ctl[slot])) continue;
-    const BLevel &F = lev[slot * kMaxDepth + depth], &C = lev[slot * kMaxDepth + depth + 1];
-    const int r = (vb - t.bstart[k]) * kCsrRows + threadIdx.x / 4;
-    const bool valid = r < F.nc;
-    const float s = row4<float, float>(F.rrp, F.rkc, F.rv, F.def, r, valid && r < F.nca, lane);
-    if (valid && lane == 0)
+#pragma unroll
+      for (int u = 0; u < U; u++)
+      {
+        const int j = b + lane + 4 * u;
+        c[u] = j < e ? __ldg(kc + j) : -1;
+        v[u] = j < e ? __ldg(a + j) : 0.f;
+      }
+    };
+    fetch();
+    if (!waited)
     {
-      C.rhs[r] = r < F.nca ? s : 0.f;
-      C.v[0][r] = 0.f;
+      CD_PDL_WAIT();
+      waited = true;
     }
+    if (stepping(p.ctl[slot]))
+      for (int base = (vb - b0) * kCsrRows; base < i1; base += kCsrRows)
+      {
+        const bool ok = i < i1;
+        const int row = r;
+        float s = 0;
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (c[u] >= 0) s += v[u] * x[c[u]];
+        for (int j = b + lane + 4 * U; j < e; j += 4) s += a[j] * x[kc[j]];
+        i += kCsrRows;
+        if (base + kCsrRows < i1) fetch();
+        s = bsum<4>(s);
+        if (!ok || lane != 0) continue;
+        if (OP == BR_JACOBI)
+          L.v[p.dst][row] = row < na ? x[row] + p.omega * (L.rhs[row] - s) / L.d32[row] : L.rhs[row];
+        else if (OP == BR_COLOR)
+          L.v[0][row] += p.omega * (L.rhs[row] - s) / L.d32[row];
+        else if (OP == BR_DEFECT)
+          L.def[row] = L.rhs[row] - s;
+        else if (OP == BR_RESTRICT)
+        {
+          C.rhs[row] = row < na ? s : 0.f;
+          C.v[0][row] = 0.f;
+        }
+        else
+          L.v[p.dst][row] += p.omega * s;
+      }
+    vb = ve;
+    k++;
   }
-}
-
-// fine v[fsrc] += damp * P coarse v[csrc] on active fine rows
-__global__ void b_prolong(BTab t, const BCtl *__restrict__ ctl, const BLevel *__restrict__ lev, int depth, int fsrc,
-                          int csrc, float damp)
-{
-  CD_PDL_ENTRY();
-  const int lane = threadIdx.x % 4;
-  for (int vb = blockIdx.x; vb < t.total; vb += gridDim.x)
-  {
-    const int k = find_item(t, vb), slot = t.item[k];
-    if (!stepping(ctl[slot])) continue;
-    const BLevel &F = lev[slot * kMaxDepth + depth], &C = lev[slot * kMaxDepth + depth + 1];
-    const int r = (vb - t.bstart[k]) * kCsrRows + threadIdx.x / 4;
-    const bool valid = r < F.na;
-    const float s = row4<float, float>(F.prp, F.pkc, F.pv, C.v[csrc], r, valid, lane);
-    if (valid && lane == 0) F.v[fsrc][r] += damp * s;
-  }
+  if (!waited) CD_PDL_WAIT();
 }
 
 // exact coarse solve on the active block (one block per instance): v[out] = A^{-1} rhs with
@@ -365,6 +411,195 @@ __global__ void b_coarse(BTab t, const BCtl *__restrict__ ctl, const BLevel *__r
       s = bsum<32>(s);
       if (lane == 0) L.v[out][r] = (float)s;
     }
+    __syncthreads();
+  }
+}
+
+// The cycle of an instance's coarse levels, from depth cta_top (at most cta_rows active rows) to
+// the exact solve and back, by one block with the iterates and right-hand sides in shared memory:
+// f of depth cta_top in, v[out] of that depth out.  The sums are those of b_rows and b_coarse.
+// These levels are bound by the number of dependent steps: a multicolour SSOR V(2,2) takes 72
+// colour classes and more per level, 2.1 us each as a grouped launch and about 1 us as a barrier
+// of one block, whose matrices (up to some 900 rows) stay in its L1; damped Jacobi takes 7
+// launches per level.  40 stationary instances with SSOR, limit on the rows: none 62.5 ms, 256
+// 55.5, 1,024 50.8, 4,096 57.1; 16 time-dependent ones with Jacobi: none 32.2 ms, 256 31.5, 1,024
+// 32.5, 4,096 38.4.
+constexpr int kCtaThreads = 512;
+inline int cta_rows(int smoother) { return smoother == 1 ? 256 : 1024; }
+constexpr size_t kCtaSmem = 100 * 1024; // two blocks per SM; the bottom level alone may take more
+
+// shared memory (floats): per level the iterate (all rows) and the right-hand side (active rows),
+// and a scratch vector for the levels above the bottom
+inline size_t cta_floats(const Hierarchy &h, int top)
+{
+  const int L = (int)h.lev.size();
+  size_t s = 0, big = 0;
+  for (int d = top; d < L; d++)
+  {
+    const Space &sp = *h.lev[L - 1 - d].sp;
+    s += (size_t)sp.n_dof + sp.n_active;
+    if (d < L - 1) big = std::max(big, (size_t)sp.n_dof);
+  }
+  return s + big;
+}
+
+__global__ void __launch_bounds__(kCtaThreads) b_cta_cycle(BTab t, const BCtl *__restrict__ ctl,
+                                                           const BLevel *__restrict__ lev, int smoother, int pre,
+                                                           int post, float omega, float damp, int out)
+{
+  CD_PDL_ENTRY();
+  extern __shared__ float csm[];
+  const int tid = threadIdx.x, lane = tid & 3, sub = tid >> 2;
+  constexpr int kRows = kCtaThreads / 4;
+  for (int k = blockIdx.x; k < t.K; k += gridDim.x)
+  {
+    const int slot = t.item[k];
+    if (!stepping(ctl[slot])) continue;
+    const BLevel *B = lev + slot * kMaxDepth;
+    const int top = B[0].cta_top, last = B[0].levels - 1;
+    if (top < 1 || top > last) continue;
+    // level vectors one after the other; the scratch vector behind them
+    int off = 0, big = 0;
+    for (int d = top; d <= last; d++)
+    {
+      off += B[d].n + B[d].na;
+      if (d < last) big = max(big, B[d].n);
+    }
+    float *tmp = csm + off;
+    for (int i = tid; i < off + big; i += kCtaThreads) csm[i] = 0.f;
+    __syncthreads();
+    // (A x)_r of active row r, Dirichlet columns carry zeros
+    auto smooth = [&](const BLevel &L, float *x, const float *f, int count, bool zero) {
+      for (int s = 0; s < count; s++)
+      {
+        if (smoother == 1)
+        {
+          const bool first = zero && s == 0;
+          for (int base = 0; base < L.na; base += kRows)
+          {
+            const int r = base + sub;
+            const bool ok = r < L.na;
+            const float v = row4<float, float>(L.rp, L.kc, L.a32, x, r, ok && !first, lane);
+            if (ok && lane == 0) tmp[r] = (first ? 0.f : x[r]) + omega * (f[r] - v) / L.d32[r];
+          }
+          __syncthreads();
+          for (int r = tid; r < L.na; r += kCtaThreads) x[r] = tmp[r];
+          __syncthreads();
+          continue;
+        }
+        // the classes of a sweep (SSOR: forward, then backward) in passes of kRows rows; the next
+        // pass's row numbers, pointers and entries are loaded while the present one is summed
+        const int nc = L.n_colors, classes = smoother == 3 ? 2 * nc : nc;
+        const int *__restrict__ list = L.color_rows, *__restrict__ ptr = L.color_ptr, *__restrict__ rp = L.rp,
+                                *__restrict__ kc = L.kc;
+        const float *__restrict__ a = L.a32, *__restrict__ d32 = L.d32;
+        constexpr int U = 8;
+        int q = 0, base = 0, end = 0, r = -1, b = 0, e = 0, c[U];
+        float v[U];
+        auto fetch = [&]() {
+          const int i = base + sub;
+          r = q < classes && i < end ? __ldg(list + i) : -1;
+          b = r >= 0 ? __ldg(rp + r) : 0;
+          e = r >= 0 ? __ldg(rp + r + 1) : 0;
+#pragma unroll
+          for (int u = 0; u < U; u++)
+          {
+            const int j = b + lane + 4 * u;
+            c[u] = j < e ? __ldg(kc + j) : -1;
+            v[u] = j < e ? __ldg(a + j) : 0.f;
+          }
+        };
+        auto open = [&]() {
+          if (q >= classes) return;
+          const int k = q < nc ? q : classes - 1 - q;
+          base = __ldg(ptr + k);
+          end = __ldg(ptr + k + 1);
+        };
+        open();
+        fetch();
+        while (q < classes)
+        {
+          const int row = r;
+          float t = 0;
+#pragma unroll
+          for (int u = 0; u < U; u++)
+            if (c[u] >= 0) t += v[u] * x[c[u]];
+          for (int j = b + lane + 4 * U; j < e; j += 4) t += a[j] * x[kc[j]];
+          const float d = row >= 0 && lane == 0 ? __ldg(d32 + row) : 1.f;
+          base += kRows;
+          const bool next = base >= end;
+          if (next)
+          {
+            q++;
+            open();
+          }
+          fetch();
+          t = bsum<4>(t);
+          if (row >= 0 && lane == 0) x[row] += omega * (f[row] - t) / d;
+          if (next) __syncthreads();
+        }
+      }
+    };
+    float *x = csm, *f = csm + B[top].n;
+    for (int i = tid; i < B[top].na; i += kCtaThreads) f[i] = B[top].rhs[i];
+    __syncthreads();
+    for (int d = top; d < last; d++)
+    {
+      const BLevel &L = B[d];
+      smooth(L, x, f, pre, true);
+      for (int base = 0; base < L.na; base += kRows)
+      {
+        const int r = base + sub;
+        const bool ok = r < L.na;
+        const float v = row4<float, float>(L.rp, L.kc, L.a32, x, r, ok, lane);
+        if (ok && lane == 0) tmp[r] = f[r] - v;
+      }
+      __syncthreads();
+      // (the scratch vector's Dirichlet entries: the defect there is zero)
+      for (int r = L.na + tid; r < L.n; r += kCtaThreads) tmp[r] = 0.f;
+      __syncthreads();
+      float *xc = f + L.na, *fc = xc + B[d + 1].n;
+      for (int base = 0; base < L.nca; base += kRows)
+      {
+        const int r = base + sub;
+        const bool ok = r < L.nca;
+        const float v = row4<float, float>(L.rrp, L.rkc, L.rv, tmp, r, ok, lane);
+        if (ok && lane == 0) fc[r] = v;
+      }
+      __syncthreads();
+      x = xc;
+      f = fc;
+    }
+    {
+      const BLevel &L = B[last];
+      const int wl = tid & 31;
+      for (int r = tid >> 5; r < L.na; r += kCtaThreads / 32)
+      {
+        double s = 0;
+        for (int j = wl; j < L.na; j += 32) s += L.cinv[(size_t)r * L.na + j] * (double)f[j];
+        s = bsum<32>(s);
+        if (wl == 0) x[r] = (float)s;
+      }
+      __syncthreads();
+    }
+    for (int d = last - 1; d >= top; d--)
+    {
+      const BLevel &L = B[d];
+      float *xf = x - L.n - L.na, *ff = xf + L.n;
+      for (int base = 0; base < L.na; base += kRows)
+      {
+        const int r = base + sub;
+        const bool ok = r < L.na;
+        const float v = row4<float, float>(L.prp, L.pkc, L.pv, x, r, ok, lane);
+        if (ok && lane == 0) xf[r] += damp * v;
+      }
+      __syncthreads();
+      smooth(L, xf, ff, post, false);
+      x = xf;
+      f = ff;
+    }
+    const BLevel &T = B[top];
+    for (int i = tid; i < T.n; i += kCtaThreads) T.v[out][i] = x[i];
     __syncthreads();
   }
 }
@@ -907,6 +1142,8 @@ static int ensure_colors(cdgpu_ctx *ctx, Hierarchy &h)
     for (int c = 0; c < nc; c++) L.h_color_ptr[c + 1] += L.h_color_ptr[c];
     std::vector<int> rows(std::max(1, s.n_active)), fill(L.h_color_ptr.begin(), L.h_color_ptr.end() - 1);
     for (int r = 0; r < s.n_active; r++) rows[fill[col[r]]++] = r;
+    // the class bounds behind the row list, for the kernels that take all classes
+    rows.insert(rows.end(), L.h_color_ptr.begin(), L.h_color_ptr.end());
     int rc = dev_alloc(ctx, &L.d_color_rows, rows.size());
     if (rc) return rc;
     CD_CUDA(ctx, cudaMemcpy(L.d_color_rows, rows.data(), sizeof(int) * rows.size(), cudaMemcpyHostToDevice));
@@ -997,9 +1234,15 @@ static int build_tables(cdgpu_ctx *ctx, Batch &b)
     if (b.inst[i].used && (b.inst[i].state == ST_RUN || b.inst[i].tcd)) b.run.push_back(i);
   if (b.tcd_graph) { cudaGraphExecDestroy(b.tcd_graph); b.tcd_graph = nullptr; }
   if (b.loop_graph) { cudaGraphExecDestroy(b.loop_graph); b.loop_graph = nullptr; }
+  // depths with grouped launches: those above the levels one block takes (all of an instance with
+  // a single level)
   int D = 0;
-  for (int i : b.run) D = std::max(D, b.inst[i].L);
+  for (int i : b.run) D = std::max(D, b.inst[i].L == 1 ? 1 : b.inst[i].cta_top);
   b.depth = D;
+  b.cta_smem = 0;
+  for (int i : b.run) b.cta_smem = std::max(b.cta_smem, b.inst[i].cta_smem);
+  if (b.cta_smem > 48 * 1024)
+    CD_CUDA(ctx, cudaFuncSetAttribute(b_cta_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.cta_smem));
   std::vector<int> pack;
   struct Pending { BTab *t; size_t item_off, bs_off; };
   std::vector<Pending> pend;
@@ -1053,14 +1296,14 @@ static int build_tables(cdgpu_ctx *ctx, Batch &b)
   std::vector<std::vector<std::vector<std::pair<int, int>>>> cpos(D);
   for (int d = 0; d < D; d++)
   {
-    auto deeper = [&](int i, int dd) { return b.inst[i].L - 1 > dd; };
+    auto deeper = [&](int i, int dd) { return b.inst[i].cta_top > dd; };
     fill(kCsrRows, nrows, deeper, d);
     add(b.smooth[d], v);
     fill(kCsrRows, [&](int i, int dd) { return level_of(i, dd + 1).sp->n_dof; }, deeper, d);
     add(b.restrict_[d], v);
     v.clear();
     for (int i : b.run)
-      if (b.inst[i].L - 1 == d) v.push_back({i, 1});
+      if (b.inst[i].L == 1 && d == 0) v.push_back({i, 1});
     add(b.coarse[d], v);
     if (b.p.smoother == 2 || b.p.smoother == 3)
     {
@@ -1135,6 +1378,12 @@ static int batch_cycle(cdgpu_ctx *ctx, Batch &b)
   const int after_pre = jac ? pre % 2 : 0, after_post = jac ? (pre + post) % 2 : 0;
   const float omega = (float)p.omega, damp = (float)p.gmg_damp;
   cudaStream_t st = ctx->stream;
+  auto rows = [&](auto kern, const BTab &t, int d, int src, int dst, float w, const int *cstart = nullptr) -> int {
+    BRowArgs a{t, b.d_ctl, b.d_lev, d, src, dst, w, cstart};
+    (void)cd_launch(kern, std::max(1, std::min(t.total, ctx->sm_count * kRowBlocks)), kNT, 0, st, a);
+    CD_LAUNCHED(ctx);
+    return CDGPU_OK;
+  };
   (void)cd_launch(b_mg_start, grid_of(ctx, b.fine_vec.total), kNT, 0, st, b.fine_vec, b.d_ctl, b.d_lev);
   CD_LAUNCHED(ctx);
   auto sweeps = [&](int d, int count, bool first_zero) -> int {
@@ -1144,9 +1393,13 @@ static int batch_cycle(cdgpu_ctx *ctx, Batch &b)
       int src = first_zero ? 0 : after_pre;
       for (int s = 0; s < count; s++)
       {
-        (void)cd_launch(b_jacobi, grid_of(ctx, t.total), kNT, 0, st, t, b.d_ctl, b.d_lev, d, src, first_zero && s == 0 ? 1 : 0,
-                                                        omega);
-        CD_LAUNCHED(ctx);
+        if (first_zero && s == 0)
+        {
+          (void)cd_launch(b_jacobi_first, grid_of(ctx, t.total), kNT, 0, st, t, b.d_ctl, b.d_lev, d, src, omega);
+          CD_LAUNCHED(ctx);
+        }
+        else if (int rc = rows(b_rows<BR_JACOBI>, t, d, src, 1 - src, omega))
+          return rc;
         src = 1 - src;
       }
     }
@@ -1160,8 +1413,7 @@ static int batch_cycle(cdgpu_ctx *ctx, Batch &b)
             const int c = pass == 0 ? q : nc - 1 - q;
             const BTab &ct = b.color[d][c];
             if (ct.K == 0) continue;
-            (void)cd_launch(b_color, grid_of(ctx, ct.total), kNT, 0, st, ct, b.d_ctl, b.d_lev, d, colour_start(ct), omega);
-            CD_LAUNCHED(ctx);
+            if (int rc = rows(b_rows<BR_COLOR>, ct, d, 0, 0, omega, colour_start(ct))) return rc;
           }
       }
     return CDGPU_OK;
@@ -1173,7 +1425,7 @@ static int batch_cycle(cdgpu_ctx *ctx, Batch &b)
       const Level *Lc = nullptr;
       int nmax = 0;
       for (int i : b.run)
-        if (b.inst[i].L - 1 == d)
+        if (b.inst[i].L == 1)
         {
           const Hierarchy &h = *ctx->mgs[b.inst[i].mg];
           Lc = &h.lev[0];
@@ -1188,24 +1440,25 @@ static int batch_cycle(cdgpu_ctx *ctx, Batch &b)
     if (b.smooth[d].K == 0) continue;
     int rc = sweeps(d, pre, true);
     if (rc) return rc;
-    (void)cd_launch(b_defect, grid_of(ctx, b.smooth[d].total), kNT, 0, st, b.smooth[d], b.d_ctl, b.d_lev, d, after_pre);
-    CD_LAUNCHED(ctx);
-    (void)cd_launch(b_restrict, grid_of(ctx, b.restrict_[d].total), kNT, 0, st, b.restrict_[d], b.d_ctl, b.d_lev, d);
+    if ((rc = rows(b_rows<BR_DEFECT>, b.smooth[d], d, after_pre, 0, 0.f))) return rc;
+    if ((rc = rows(b_rows<BR_RESTRICT>, b.restrict_[d], d, 0, 0, 0.f))) return rc;
+  }
+  if (b.cta_smem > 0)
+  {
+    (void)cd_launch(b_cta_cycle, grid_of(ctx, b.items.K), kCtaThreads, b.cta_smem, st, b.items, b.d_ctl, b.d_lev,
+                    p.smoother, pre, post, omega, damp, after_post);
     CD_LAUNCHED(ctx);
   }
-  for (int d = D - 2; d >= 0; d--)
+  for (int d = D - 1; d >= 0; d--)
   {
     if (b.smooth[d].K == 0) continue;
-    (void)cd_launch(b_prolong, grid_of(ctx, b.smooth[d].total), kNT, 0, st, b.smooth[d], b.d_ctl, b.d_lev, d, after_pre,
-                                                               after_post, damp);
-    CD_LAUNCHED(ctx);
+    if (int rc = rows(b_rows<BR_PROLONG>, b.smooth[d], d, after_post, after_pre, damp)) return rc;
     if (jac)
     {
       int src = after_pre;
       for (int s = 0; s < post; s++)
       {
-        (void)cd_launch(b_jacobi, grid_of(ctx, b.smooth[d].total), kNT, 0, st, b.smooth[d], b.d_ctl, b.d_lev, d, src, 0, omega);
-        CD_LAUNCHED(ctx);
+        if (int rc = rows(b_rows<BR_JACOBI>, b.smooth[d], d, src, 1 - src, omega)) return rc;
         src = 1 - src;
       }
     }
@@ -1755,6 +2008,12 @@ static int submit_impl(cdgpu_ctx *ctx, Batch &b, int mg_id, const cdgpu_coeffs *
   in.used = true;
   in.mg = mg_id;
   in.L = L;
+  // the levels one block takes: from the first depth below the finest of few enough rows on
+  in.cta_top = L == 1 ? 0 : L - 1;
+  while (in.cta_top > 1 && h.lev[L - in.cta_top].sp->n_active <= cta_rows(b.p.smoother) &&
+         cta_floats(h, in.cta_top - 1) * sizeof(float) <= kCtaSmem)
+    in.cta_top--;
+  in.cta_smem = L == 1 ? 0 : cta_floats(h, in.cta_top) * sizeof(float);
   const int m = b.m;
   {
     // the instance's arrays in one allocation (the estimate of instance_bytes plus the
@@ -1829,6 +2088,11 @@ static int submit_impl(cdgpu_ctx *ctx, Batch &b, int mg_id, const cdgpu_coeffs *
     B.kc = s.d_kcol;
     B.dirst = s.d_dir_start;
     B.color_rows = Lv.d_color_rows;
+    if (Lv.n_colors >= 0)
+    {
+      B.n_colors = Lv.n_colors;
+      B.color_ptr = Lv.d_color_rows + std::max(1, s.n_active);
+    }
     B.a32 = a32;
     B.d32 = d32;
     B.a64 = a64;
@@ -1908,6 +2172,8 @@ static int submit_impl(cdgpu_ctx *ctx, Batch &b, int mg_id, const cdgpu_coeffs *
     }
     B.cinv = cinv;
   }
+  lv[0].cta_top = in.cta_top;
+  lv[0].levels = L;
   // pageable host sources: the copy is staged before the call returns.  Assembly errors
   // (a cell coupling missing from the pattern) are collected at the next advance.
   CD_CUDA(ctx, cudaMemcpyAsync(b.d_lev + (size_t)sl * kMaxDepth, lv.data(), sizeof(BLevel) * kMaxDepth,
