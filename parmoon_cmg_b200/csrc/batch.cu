@@ -26,6 +26,7 @@
 #include <cstring>
 
 #include "internal.h"
+#include "warp.cuh"
 
 namespace
 {
@@ -33,6 +34,7 @@ constexpr int kMaxDepth = 12;
 constexpr int kNT = 256;
 constexpr int kCsrRows = 64;  // rows per virtual block of the CSR kernels (4 threads per row)
 constexpr int kVecRows = 256; // rows per virtual block of the vector kernels
+constexpr int kGsRows = 1024; // rows per virtual block of the Gram-Schmidt passes
 constexpr int kMaxM = 32;
 constexpr int kSlots = 33;
 
@@ -120,7 +122,7 @@ struct Batch
   // tables of the current running set
   std::vector<int> run;
   int depth = 0;
-  BTab fine_vec, fine_csr, items;
+  BTab fine_vec, fine_gs, fine_csr, items;
   BTab tcd_csr, tcd_items; // every time-dependent instance, running or idle
   cudaGraphExec_t tcd_graph = nullptr;
   int tcd_graph_k = 0;
@@ -174,6 +176,22 @@ __device__ __forceinline__ int find_item(const BTab &t, int vb)
   return lo;
 }
 
+// the item of virtual block vb, by a whole warp: 32 bounds at a time
+__device__ __forceinline__ int find_item_warp(const BTab &t, int vb)
+{
+  const int lane = threadIdx.x & 31;
+  int lo = 0, n = t.K;
+  while (n > 1)
+  {
+    const int step = (n + 31) >> 5, i = lo + lane * step;
+    const unsigned m = __ballot_sync(0xffffffffu, i < lo + n && __ldg(t.bstart + i) <= vb);
+    const int c = __popc(m) - 1;
+    n = min(step, n - c * step);
+    lo += c * step;
+  }
+  return lo;
+}
+
 template <int G, typename T> __device__ __forceinline__ T bsum(T v)
 {
 #pragma unroll
@@ -207,60 +225,92 @@ __device__ __forceinline__ TX row4(const int *__restrict__ rp, const int *__rest
   return bsum<4>(s);
 }
 
-__device__ __forceinline__ bool stepping(const BCtl &c) { return c.state == ST_RUN && c.action == A_STEP; }
+// in an Arnoldi step, the first one of a restart cycle (V_0 not yet scaled before b_mg_start) included
+__device__ __forceinline__ bool stepping(const BCtl &c)
+{
+  return c.state == ST_RUN && (c.action == A_STEP || c.action == A_SCALE0);
+}
 
 // ---------------------------------------------------------------------------
 // multigrid kernels (FP32)
 // ---------------------------------------------------------------------------
-// zero start + Dirichlet nodes on depth 0 from the current basis vector V_j
-__global__ void b_mg_start(BTab t, const BCtl *__restrict__ ctl, const BLevel *__restrict__ lev)
+// Start of a cycle from the current basis vector V_j (scaled here when it is the residual of a
+// restart): right-hand side and zero start with the Dirichlet values of depth 0
+__global__ void __launch_bounds__(kNT) b_mg_start(BTab t, const BCtl *__restrict__ ctl, const BLevel *__restrict__ lev)
 {
   CD_PDL_ENTRY();
-  for (int vb = blockIdx.x; vb < t.total; vb += gridDim.x)
+  const int v1 = (int)((long)t.total * (blockIdx.x + 1) / gridDim.x);
+  int vb = (int)((long)t.total * blockIdx.x / gridDim.x);
+  for (int k = find_item_warp(t, vb); vb < v1; k++)
   {
-    const int k = find_item(t, vb), slot = t.item[k];
+    const int slot = __ldg(t.item + k), b0 = __ldg(t.bstart + k), ve = min(v1, __ldg(t.bstart + k + 1));
     const BCtl &c = ctl[slot];
-    if (!stepping(c)) continue;
-    const BLevel &L = lev[slot * kMaxDepth];
-    const int r = (vb - t.bstart[k]) * kVecRows + threadIdx.x;
-    if (r >= L.n) continue;
-    const float v = (float)c.V[(size_t)c.j * c.n + r];
-    L.rhs[r] = v;
-    L.v[0][r] = r < L.na ? 0.f : v;
+    if (stepping(c))
+    {
+      const BLevel &L = lev[slot * kMaxDepth];
+      double *V = c.V + (size_t)c.j * c.n;
+      const bool scale = c.action == A_SCALE0;
+      const double beta = c.beta;
+      const int n = c.n, na = L.na, r1 = min(n, (ve - b0) * kVecRows);
+      float *f = L.rhs, *x = L.v[0];
+      for (int r = (vb - b0) * kVecRows + threadIdx.x; r < r1; r += kNT)
+      {
+        double d = V[r];
+        if (scale)
+        {
+          d /= beta;
+          V[r] = d;
+        }
+        const float v = (float)d;
+        f[r] = v;
+        x[r] = r < na ? 0.f : v;
+      }
+    }
+    vb = ve;
   }
 }
 
-// First damped Jacobi sweep of depth `depth` when the active part of v[src] is zero: only Dirichlet
-// columns (from dirst) contribute
-__global__ void b_jacobi_first(BTab t, const BCtl *__restrict__ ctl, const BLevel *__restrict__ lev, int depth, int src,
-                               float omega)
+// First damped Jacobi sweep of depth 0, from v[0] (zero but for the Dirichlet values) into v[1]:
+// only Dirichlet columns (from dirst) contribute
+__global__ void __launch_bounds__(kNT) b_jacobi_first(BTab t, const BCtl *__restrict__ ctl,
+                                                      const BLevel *__restrict__ lev, float omega)
 {
   CD_PDL_ENTRY();
-  const int lane = threadIdx.x % 4;
-  for (int vb = blockIdx.x; vb < t.total; vb += gridDim.x)
+  const int v1 = (int)((long)t.total * (blockIdx.x + 1) / gridDim.x);
+  int vb = (int)((long)t.total * blockIdx.x / gridDim.x);
+  for (int k = find_item_warp(t, vb); vb < v1; k++)
   {
-    const int k = find_item(t, vb), slot = t.item[k];
-    if (!stepping(ctl[slot])) continue;
-    const BLevel &L = lev[slot * kMaxDepth + depth];
-    const int r = (vb - t.bstart[k]) * kCsrRows + threadIdx.x / 4;
-    if (r >= L.n || lane != 0) continue;
-    const float *x = L.v[src];
-    if (r >= L.na)
-      L.v[1 - src][r] = L.rhs[r];
-    else
+    const int slot = __ldg(t.item + k), b0 = __ldg(t.bstart + k), ve = min(v1, __ldg(t.bstart + k + 1));
+    const BLevel &L = lev[slot * kMaxDepth];
+    if (stepping(ctl[slot]) && L.levels > 1) // a single level has the exact solve alone
     {
-      float s = L.rhs[r];
-      for (int j = L.dirst[r]; j < L.rp[r + 1]; j++) s -= L.a32[j] * x[L.kc[j]];
-      L.v[1 - src][r] = omega * s / L.d32[r];
+      const int na = L.na, r1 = min(L.n, (ve - b0) * kVecRows);
+      const int *__restrict__ rp = L.rp, *__restrict__ dirst = L.dirst;
+      const float *x = L.v[0], *f = L.rhs, *__restrict__ d32 = L.d32;
+      float *y = L.v[1];
+      for (int r = (vb - b0) * kVecRows + threadIdx.x; r < r1; r += kNT)
+      {
+        float s = f[r];
+        if (r < na)
+        {
+          const int e = __ldg(rp + r + 1);
+          for (int j = __ldg(dirst + r); j < e; j++) s -= L.a32[j] * x[L.kc[j]];
+          s = omega * s / __ldg(d32 + r);
+        }
+        y[r] = s;
+      }
     }
+    vb = ve;
   }
 }
 
 // The grouped row operations of the cycle, y_r = epilogue((A x)_r) with 4 threads per row:
-//   BR_JACOBI    v[dst] = v[src] + omega D^{-1} (f - A v[src]), Dirichlet rows f
+//   BR_JACOBI    v[dst] = v[src] + omega D^{-1} (f - A v[src]), Dirichlet rows f; dst 2: the cycle's
+//                result Z_j in FP64
 //   BR_COLOR     one colour class of an SOR sweep, in place on v[0]
 //   BR_DEFECT    def = f - A v[src]
-//   BR_RESTRICT  coarse f = R def on active coarse rows (zero elsewhere), coarse v[0] = 0
+//   BR_RESTRICT  coarse f = R def on active coarse rows (zero elsewhere); coarse v[0] = 0, or with
+//                omega the first Jacobi sweep from zero, coarse v[1] = omega D^{-1} f
 //   BR_PROLONG   v[dst] += omega P (coarse v[src]) on active rows
 // A block takes a contiguous range of virtual blocks, so it looks an instance up once and then
 // walks its rows, the next rows' pointers and entries loaded while the present ones are summed;
@@ -280,22 +330,6 @@ struct BRowArgs
   float omega;
   const int *cstart; // colour class: first position of item k in its level's row list, K + k: count
 };
-
-// the item of virtual block vb, by a whole warp: 32 bounds at a time
-__device__ __forceinline__ int find_item_warp(const BTab &t, int vb)
-{
-  const int lane = threadIdx.x & 31;
-  int lo = 0, n = t.K;
-  while (n > 1)
-  {
-    const int step = (n + 31) >> 5, i = lo + lane * step;
-    const unsigned m = __ballot_sync(0xffffffffu, i < lo + n && __ldg(t.bstart + i) <= vb);
-    const int c = __popc(m) - 1;
-    n = min(step, n - c * step);
-    lo += c * step;
-  }
-  return lo;
-}
 
 // Blocks per SM (40 stationary instances with SSOR and 16 time-dependent ones with Jacobi, solve
 // phases included: 62.5 and 32.2 ms with 4, 66.9 and 31.7 with 5, 73.5 and 36.2 with 6, whose
@@ -346,7 +380,9 @@ template <int OP> __global__ void __launch_bounds__(kNT, kRowBlocks) b_rows(cons
       CD_PDL_WAIT();
       waited = true;
     }
-    if (stepping(p.ctl[slot]))
+    const BCtl &ctl = p.ctl[slot];
+    double *Z = OP == BR_JACOBI && p.dst == 2 ? ctl.Z + (size_t)ctl.j * ctl.n : nullptr;
+    if (stepping(ctl))
       for (int base = (vb - b0) * kCsrRows; base < i1; base += kCsrRows)
       {
         const bool ok = i < i1;
@@ -361,7 +397,13 @@ template <int OP> __global__ void __launch_bounds__(kNT, kRowBlocks) b_rows(cons
         s = bsum<4>(s);
         if (!ok || lane != 0) continue;
         if (OP == BR_JACOBI)
-          L.v[p.dst][row] = row < na ? x[row] + p.omega * (L.rhs[row] - s) / L.d32[row] : L.rhs[row];
+        {
+          const float y = row < na ? x[row] + p.omega * (L.rhs[row] - s) / L.d32[row] : L.rhs[row];
+          if (p.dst == 2)
+            Z[row] = (double)y;
+          else
+            L.v[p.dst][row] = y;
+        }
         else if (OP == BR_COLOR)
           L.v[0][row] += p.omega * (L.rhs[row] - s) / L.d32[row];
         else if (OP == BR_DEFECT)
@@ -369,7 +411,10 @@ template <int OP> __global__ void __launch_bounds__(kNT, kRowBlocks) b_rows(cons
         else if (OP == BR_RESTRICT)
         {
           C.rhs[row] = row < na ? s : 0.f;
-          C.v[0][row] = 0.f;
+          if (p.omega == 0.f)
+            C.v[0][row] = 0.f;
+          else
+            C.v[1][row] = row < na ? p.omega * s / C.d32[row] : 0.f;
         }
         else
           L.v[p.dst][row] += p.omega * s;
@@ -604,156 +649,232 @@ __global__ void __launch_bounds__(kCtaThreads) b_cta_cycle(BTab t, const BCtl *_
   }
 }
 
-// Z_j = v[src] of depth 0, in FP64
-__global__ void b_mg_finish(BTab t, const BCtl *__restrict__ ctl, const BLevel *__restrict__ lev, int src)
+// Z_j = v[src] of depth 0, in FP64 (single: only for instances of a single level)
+__global__ void __launch_bounds__(kNT) b_mg_finish(BTab t, const BCtl *__restrict__ ctl,
+                                                   const BLevel *__restrict__ lev, int src, int single)
 {
   CD_PDL_ENTRY();
-  for (int vb = blockIdx.x; vb < t.total; vb += gridDim.x)
+  const int v1 = (int)((long)t.total * (blockIdx.x + 1) / gridDim.x);
+  int vb = (int)((long)t.total * blockIdx.x / gridDim.x);
+  for (int k = find_item_warp(t, vb); vb < v1; k++)
   {
-    const int k = find_item(t, vb), slot = t.item[k];
+    const int slot = __ldg(t.item + k), b0 = __ldg(t.bstart + k), ve = min(v1, __ldg(t.bstart + k + 1));
     const BCtl &c = ctl[slot];
-    if (!stepping(c)) continue;
     const BLevel &L = lev[slot * kMaxDepth];
-    const int r = (vb - t.bstart[k]) * kVecRows + threadIdx.x;
-    if (r < L.n) c.Z[(size_t)c.j * c.n + r] = (double)L.v[src][r];
+    if (stepping(c) && !(single && L.levels > 1))
+    {
+      const int n = c.n, r1 = min(n, (ve - b0) * kVecRows);
+      const float *x = L.v[src];
+      double *Z = c.Z + (size_t)c.j * n;
+      for (int r = (vb - b0) * kVecRows + threadIdx.x; r < r1; r += kNT) Z[r] = (double)x[r];
+    }
+    vb = ve;
   }
 }
 
 // ---------------------------------------------------------------------------
 // FGMRES kernels (FP64)
 // ---------------------------------------------------------------------------
-// w = A Z_j (stepping instances), or for restarting instances V_0 = b - A x with per-block
-// partial sums of its square
-__global__ void b_matvec(BTab t, const BCtl *__restrict__ ctl, int restart_phase, double *__restrict__ partial)
+// The sums of an instance are taken over its own blocks of rows (kGsRows for the Gram-Schmidt
+// passes, kCsrRows for the restart residual) and added in an order that depends on their number
+// alone, so an instance's results do not depend on what else runs.  Partial sum s of virtual block
+// vb is partial[s * total + vb]; the kernel that needs a sum adds the instance's partials itself,
+// each of its blocks the same ones in the same order, so no kernel only reduces.
+
+// blocks' partial sums of up to `slots` sums of an instance with virtual blocks [b0, b1) into
+// out[]: a warp takes up to 5 slots at once, its lanes the blocks; ends with a barrier
+__device__ __forceinline__ void b_gather(const double *__restrict__ partial, int total, int b0, int b1, int slots,
+                                         double *out)
+{
+  constexpr int W = kNT / 32, S = (kSlots + W - 1) / W;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double t[S];
+#pragma unroll
+  for (int s = 0; s < S; s++) t[s] = 0;
+#pragma unroll 2
+  for (int b = b0 + lane; b < b1; b += 32)
+#pragma unroll
+    for (int s = 0; s < S; s++)
+      if (warp + s * W < slots) t[s] += __ldcg(partial + (size_t)(warp + s * W) * total + b);
+#pragma unroll
+  for (int s = 0; s < S; s++)
+  {
+    if (warp + s * W >= slots) break;
+    const double v = bsum<32>(t[s]);
+    if (lane == 0) out[warp + s * W] = v;
+  }
+  __syncthreads();
+}
+
+// w = A Z_j (stepping instances), or for restarting instances (RESTART) V_0 = b - A x with
+// partial sums of its square; walks rows like b_rows
+template <bool RESTART>
+__global__ void __launch_bounds__(kNT, 3) b_matvec(BTab t, const BCtl *__restrict__ ctl, double *__restrict__ partial)
 {
   CD_PDL_ENTRY();
   __shared__ double red[kNT / 32];
-  const int lane = threadIdx.x % 4;
-  for (int vb = blockIdx.x; vb < t.total; vb += gridDim.x)
+  constexpr int U = 8;
+  const int lane = threadIdx.x & 3, sub = threadIdx.x >> 2;
+  const int v1 = (int)((long)t.total * (blockIdx.x + 1) / gridDim.x);
+  int vb = (int)((long)t.total * blockIdx.x / gridDim.x);
+  for (int k = find_item_warp(t, vb); vb < v1; k++)
   {
-    const int k = find_item(t, vb), slot = t.item[k];
+    const int slot = __ldg(t.item + k), b0 = __ldg(t.bstart + k), ve = min(v1, __ldg(t.bstart + k + 1));
     const BCtl &c = ctl[slot];
-    const bool act = restart_phase ? (c.state == ST_RUN && c.action == A_START) : stepping(c);
-    if (!act) continue;
-    const int r = (vb - t.bstart[k]) * kCsrRows + threadIdx.x / 4;
-    const bool valid = r < c.n;
-    const double *x = restart_phase ? c.x : c.Z + (size_t)c.j * c.n;
-    const double s = row4<double, double>(c.rp, c.kc, c.a64, x, r, valid, lane);
-    double sq = 0;
-    if (valid && lane == 0)
+    if (!(RESTART ? c.state == ST_RUN && c.action == A_START : stepping(c)))
     {
-      if (restart_phase)
-      {
-        const double v = c.b[r] - s;
-        c.V[r] = v;
-        sq = v * v;
-      }
-      else
-        c.w[r] = s;
+      vb = ve;
+      continue;
     }
-    if (restart_phase)
-    {
-      sq = bsum<32>(sq);
-      if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = sq;
-      __syncthreads();
-      if (threadIdx.x == 0)
+    const int *__restrict__ rp = c.rp, *__restrict__ kc = c.kc;
+    const double *__restrict__ a = c.a64, *__restrict__ x = RESTART ? c.x : c.Z + (size_t)c.j * c.n;
+    const double *f = c.b;
+    double *y = RESTART ? c.V : c.w;
+    const int r1 = min(c.n, (ve - b0) * kCsrRows);
+    int r = (vb - b0) * kCsrRows + sub, b = 0, e = 0, col[U];
+    double v[U];
+    auto fetch = [&]() {
+      b = r < r1 ? __ldg(rp + r) : 0;
+      e = r < r1 ? __ldg(rp + r + 1) : 0;
+#pragma unroll
+      for (int u = 0; u < U; u++)
       {
-        double tot = 0;
-        for (int w = 0; w < kNT / 32; w++) tot += red[w];
-        partial[(size_t)vb * kSlots] = tot;
+        const int j = b + lane + 4 * u;
+        col[u] = j < e ? __ldg(kc + j) : -1;
+        v[u] = j < e ? __ldg(a + j) : 0.0;
       }
-      __syncthreads();
-    }
-  }
-}
-
-// one fused classical Gram-Schmidt pass over V_0..V_j: mode 0 dots, 1 axpy (dots1) + dots,
-// 2 axpy (dots2) + norm; per-virtual-block partials in partial[vb * 33 + t]
-__global__ void b_gs(BTab t, const BCtl *__restrict__ ctl, int mode, double *__restrict__ partial)
-{
-  CD_PDL_ENTRY();
-  __shared__ double red[kNT / 32][kSlots];
-  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  for (int vb = blockIdx.x; vb < t.total; vb += gridDim.x)
-  {
-    const int k = find_item(t, vb), slot = t.item[k];
-    const BCtl &c = ctl[slot];
-    if (!stepping(c)) continue;
-    const int kk = c.j + 1, n = c.n;
-    const int r = (vb - t.bstart[k]) * kVecRows + threadIdx.x;
-    const bool valid = r < n;
-    double w = valid ? c.w[r] : 0.0;
-    if (mode > 0)
+    };
+    fetch();
+    for (; vb < ve; vb++)
     {
-      const double *cf = mode == 1 ? c.dots1 : c.dots2;
-      if (valid)
-      {
-        for (int q = 0; q < kk; q++) w -= cf[q] * c.V[(size_t)q * n + r];
-        c.w[r] = w;
-      }
-    }
-    if (mode == 2)
-    {
-      double sq = bsum<32>(w * w);
-      if (lane == 0) red[warp][0] = sq;
-      __syncthreads();
-      if (threadIdx.x == 0)
-      {
-        double tot = 0;
-        for (int q = 0; q < kNT / 32; q++) tot += red[q][0];
-        partial[(size_t)vb * kSlots] = tot;
-      }
-    }
-    else
-    {
-      for (int q = 0; q < kk; q++)
-      {
-        double p = bsum<32>(valid ? w * c.V[(size_t)q * n + r] : 0.0);
-        if (lane == 0) red[warp][q] = p;
-      }
-      __syncthreads();
-      if (threadIdx.x < kk)
-      {
-        double tot = 0;
-        for (int q = 0; q < kNT / 32; q++) tot += red[q][threadIdx.x];
-        partial[(size_t)vb * kSlots + threadIdx.x] = tot;
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// per-instance sums of the partials of table t into ctl (which 0: dots1, 1: dots2, 2: nrm2);
-// one block per instance, fixed order
-__global__ void b_reduce(BTab t, BCtl *__restrict__ ctl, int which, int restart_phase,
-                         const double *__restrict__ partial)
-{
-  CD_PDL_ENTRY();
-  __shared__ double red[kNT / 32];
-  for (int k = blockIdx.x; k < t.K; k += gridDim.x)
-  {
-    const int slot = t.item[k];
-    BCtl &c = ctl[slot];
-    const bool act = restart_phase ? (c.state == ST_RUN && c.action == A_START) : stepping(c);
-    if (!act) continue;
-    const int nslots = which == 2 ? 1 : c.j + 1;
-    const int b0 = t.bstart[k], b1 = t.bstart[k + 1];
-    for (int q = 0; q < nslots; q++)
-    {
+      const int row = r;
       double s = 0;
-      for (int b = b0 + threadIdx.x; b < b1; b += blockDim.x) s += partial[(size_t)b * kSlots + q];
-      s = bsum<32>(s);
-      if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = s;
-      __syncthreads();
-      if (threadIdx.x == 0)
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (col[u] >= 0) s += v[u] * x[col[u]];
+      for (int j = b + lane + 4 * U; j < e; j += 4) s += a[j] * x[kc[j]];
+      r += kCsrRows;
+      if (vb + 1 < ve) fetch();
+      s = bsum<4>(s);
+      double sq = 0;
+      if (row < r1 && lane == 0)
       {
-        double tot = 0;
-        for (int w = 0; w < kNT / 32; w++) tot += red[w];
-        if (which == 0) c.dots1[q] = tot;
-        else if (which == 1) c.dots2[q] = tot;
-        else c.nrm2 = tot;
+        if (RESTART)
+        {
+          const double d = f[row] - s;
+          y[row] = d;
+          sq = d * d;
+        }
+        else
+          y[row] = s;
       }
-      __syncthreads();
+      if (RESTART)
+      {
+        sq = bsum<32>(sq);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sq;
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+          double tot = 0;
+          for (int w = 0; w < kNT / 32; w++) tot += red[w];
+          partial[vb] = tot;
+        }
+        __syncthreads();
+      }
+    }
+  }
+}
+
+// One classical Gram-Schmidt pass over the kk <= 8 G basis vectors for the rows of a virtual block:
+// (AXPY) w -= sum_q h_q V_q first, then the sums w . V_q and (AXPY) ||w||^2, kept per block
+template <int G, bool AXPY>
+__device__ __forceinline__ void b_gs_rows(const BCtl &c, int kk, const double *h, int r0, int vb, int total,
+                                          double *__restrict__ partial, double (&red)[kNT / 32][kSlots])
+{
+  constexpr int K = 8 * G, R = G == 1 ? 4 : G == 2 ? 2 : 1;
+  const int n = c.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double *__restrict__ V = c.V;
+  double *w = c.w;
+  double acc[K], sq = 0;
+#pragma unroll
+  for (int q = 0; q < K; q++) acc[q] = 0;
+  for (int p = 0; p < kGsRows / kNT; p += R)
+  {
+    double y[R][K], wv[R];
+#pragma unroll
+    for (int u = 0; u < R; u++)
+    {
+      const int r = r0 + (p + u) * kNT + threadIdx.x;
+      wv[u] = r < n ? w[r] : 0.0;
+#pragma unroll
+      for (int q = 0; q < K; q++) y[u][q] = r < n && q < kk ? __ldg(V + (size_t)q * n + r) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < R; u++)
+    {
+      const int r = r0 + (p + u) * kNT + threadIdx.x;
+      if (AXPY)
+      {
+#pragma unroll
+        for (int q = 0; q < K; q++)
+          if (q < kk) wv[u] -= h[q] * y[u][q];
+        if (r < n) w[r] = wv[u];
+        sq += wv[u] * wv[u];
+      }
+#pragma unroll
+      for (int q = 0; q < K; q++) acc[q] += wv[u] * y[u][q];
+    }
+  }
+  const double s = warp_sums<K>(acc);
+  if (lane < kk) red[warp][lane] = s;
+  if (AXPY)
+  {
+    sq = bsum<32>(sq);
+    if (lane == 0) red[warp][kk] = sq;
+  }
+  __syncthreads();
+  if (threadIdx.x < kk + (AXPY ? 1 : 0))
+  {
+    double tot = 0;
+    for (int g = 0; g < kNT / 32; g++) tot += red[g][threadIdx.x];
+    partial[(size_t)threadIdx.x * total + vb] = tot;
+  }
+  __syncthreads();
+}
+
+// AXPY false: partial sums of h1 = V^T w in p2; true: h1 from p1 (kept in ctl.dots1), w -= V h1,
+// partial sums of h2 = V^T w and ||w||^2 in p2
+template <bool AXPY>
+__global__ void __launch_bounds__(kNT, 2) b_gs(BTab t, BCtl *__restrict__ ctl, const double *__restrict__ p1,
+                                               double *__restrict__ p2)
+{
+  CD_PDL_ENTRY();
+  __shared__ double red[kNT / 32][kSlots], h[kSlots];
+  const int v1 = (int)((long)t.total * (blockIdx.x + 1) / gridDim.x);
+  int vb = (int)((long)t.total * blockIdx.x / gridDim.x);
+  for (int k = find_item_warp(t, vb); vb < v1; k++)
+  {
+    const int slot = __ldg(t.item + k), b0 = __ldg(t.bstart + k), b1 = __ldg(t.bstart + k + 1), ve = min(v1, b1);
+    BCtl &c = ctl[slot];
+    if (!stepping(c))
+    {
+      vb = ve;
+      continue;
+    }
+    const int kk = c.j + 1;
+    if (AXPY)
+    {
+      __syncthreads(); // the previous instance's coefficients are no longer read
+      b_gather(p1, t.total, b0, b1, kk, h);
+      if (vb == b0 && threadIdx.x < kk) c.dots1[threadIdx.x] = h[threadIdx.x];
+    }
+    for (; vb < ve; vb++)
+    {
+      const int r0 = (vb - b0) * kGsRows;
+      if (kk <= 8) b_gs_rows<1, AXPY>(c, kk, h, r0, vb, t.total, p2, red);
+      else if (kk <= 16) b_gs_rows<2, AXPY>(c, kk, h, r0, vb, t.total, p2, red);
+      else if (kk <= 24) b_gs_rows<3, AXPY>(c, kk, h, r0, vb, t.total, p2, red);
+      else b_gs_rows<4, AXPY>(c, kk, h, r0, vb, t.total, p2, red);
     }
   }
 }
@@ -783,24 +904,49 @@ __device__ void d_solve_y(BCtl &c, int k)
   }
 }
 
-// Hessenberg column j, rotations, residual, stopping tests (FgmresIte.C:410-530)
-__global__ void b_givens(BTab t, BCtl *__restrict__ ctl, int maxit, int minit, double div_factor)
+// Hessenberg column j, rotations, residual, stopping tests (FgmresIte.C:410-530); one block per
+// instance, which first adds up h2 = V^T w and ||w - V h2||^2 = ||w||^2 - ||h2||^2 (V orthonormal)
+__global__ void __launch_bounds__(kNT) b_givens(BTab t, BCtl *__restrict__ ctl, const double *__restrict__ partial,
+                                                int maxit, int minit, double div_factor)
 {
   CD_PDL_ENTRY();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < t.K; k += gridDim.x * blockDim.x)
+  __shared__ double d2[kSlots], h[kSlots + 1], cs[kMaxM], sn[kMaxM];
+  for (int k = blockIdx.x; k < t.K; k += gridDim.x)
   {
     BCtl &c = ctl[t.item[k]];
     if (!stepping(c)) continue;
     const int j = c.j, ld = c.m + 1;
-    double *h = c.H + (size_t)j * ld;
-    for (int q = 0; q <= j; q++) h[q] = c.dots1[q] + c.dots2[q];
-    const double hn = sqrt(c.nrm2);
-    h[j + 1] = hn;
-    c.hn = hn;
-    for (int q = 0; q < j; q++) d_app_rot(h[q], h[q + 1], c.cs[q], c.sn[q]);
-    d_gen_rot(h[j], h[j + 1], c.cs[j], c.sn[j]);
-    d_app_rot(h[j], h[j + 1], c.cs[j], c.sn[j]);
-    d_app_rot(c.s[j], c.s[j + 1], c.cs[j], c.sn[j]);
+    double *H = c.H + (size_t)j * ld;
+    __syncthreads();
+    b_gather(partial, t.total, t.bstart[k], t.bstart[k + 1], j + 2, d2);
+    if (threadIdx.x <= j)
+    {
+      c.dots2[threadIdx.x] = d2[threadIdx.x];
+      h[threadIdx.x] = c.dots1[threadIdx.x] + d2[threadIdx.x];
+      if (threadIdx.x < j)
+      {
+        cs[threadIdx.x] = c.cs[threadIdx.x];
+        sn[threadIdx.x] = c.sn[threadIdx.x];
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+      double n2 = d2[j + 1];
+      for (int q = 0; q <= j; q++) n2 -= d2[q] * d2[q];
+      const double hn = sqrt(n2 > 0.0 ? n2 : 0.0);
+      h[j + 1] = hn;
+      c.hn = hn;
+      for (int q = 0; q < j; q++) d_app_rot(h[q], h[q + 1], cs[q], sn[q]);
+      d_gen_rot(h[j], h[j + 1], c.cs[j], c.sn[j]);
+      d_app_rot(h[j], h[j + 1], c.cs[j], c.sn[j]);
+      d_app_rot(c.s[j], c.s[j + 1], c.cs[j], c.sn[j]);
+    }
+    __syncthreads();
+    if (threadIdx.x <= j + 1) H[threadIdx.x] = h[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x != 0) continue;
+    const double hn = c.hn;
     c.res = fabs(c.s[j + 1]);
     c.its++;
     if (c.its >= minit && c.res < c.tol)
@@ -833,25 +979,36 @@ __global__ void b_givens(BTab t, BCtl *__restrict__ ctl, int maxit, int minit, d
   }
 }
 
-// V_{j+1} = w / h_{j+1,j} (A_NEXT), or x += Z y (A_UPD_*)
-__global__ void b_next_update(BTab t, const BCtl *__restrict__ ctl)
+// V_{j+1} = (w - V h2) / h_{j+1,j} (A_NEXT), or x += Z y (A_UPD_*)
+__global__ void __launch_bounds__(kNT) b_next_update(BTab t, const BCtl *__restrict__ ctl)
 {
   CD_PDL_ENTRY();
-  for (int vb = blockIdx.x; vb < t.total; vb += gridDim.x)
+  const int v1 = (int)((long)t.total * (blockIdx.x + 1) / gridDim.x);
+  int vb = (int)((long)t.total * blockIdx.x / gridDim.x);
+  for (int k = find_item_warp(t, vb); vb < v1; k++)
   {
-    const int k = find_item(t, vb), slot = t.item[k];
+    const int slot = __ldg(t.item + k), b0 = __ldg(t.bstart + k), ve = min(v1, __ldg(t.bstart + k + 1));
     const BCtl &c = ctl[slot];
-    if (c.state != ST_RUN) continue;
-    const int r = (vb - t.bstart[k]) * kVecRows + threadIdx.x;
-    if (r >= c.n) continue;
-    if (c.action == A_NEXT)
-      c.V[(size_t)(c.j + 1) * c.n + r] = c.w[r] / c.hn;
-    else if (c.action == A_UPD_DONE || c.action == A_UPD_RESTART)
+    const bool next = c.action == A_NEXT;
+    const int n = c.n, r1 = min(n, (ve - b0) * kVecRows);
+    if (c.state == ST_RUN && (next || c.action == A_UPD_DONE || c.action == A_UPD_RESTART))
     {
-      double s = 0;
-      for (int q = 0; q <= c.last; q++) s += c.y[q] * c.Z[(size_t)q * c.n + r];
-      c.x[r] += s;
+      // out = in + sum_q cf_q B_q: w - V h2, or x + Z y
+      const double *__restrict__ B = next ? c.V : c.Z, *cf = next ? c.dots2 : c.y;
+      const int kk = next ? c.j + 1 : c.last + 1;
+      const double inv = next ? 1.0 / c.hn : 1.0;
+      for (int r = (vb - b0) * kVecRows + threadIdx.x; r < r1; r += kNT)
+      {
+        double s = 0;
+#pragma unroll 8
+        for (int q = 0; q < kk; q++) s += cf[q] * __ldg(B + (size_t)q * n + r);
+        if (next)
+          c.V[(size_t)(c.j + 1) * n + r] = inv * (c.w[r] - s);
+        else
+          c.x[r] += s;
+      }
     }
+    vb = ve;
   }
 }
 
@@ -896,15 +1053,21 @@ __global__ void b_loop_budget(int *__restrict__ loop, int iterations)
   loop[0] = iterations;
 }
 
-// restart: beta = ||b - A x||, stopping test on it, s = (beta, 0, ...), j = 0
-__global__ void b_restart(BTab t, BCtl *__restrict__ ctl, int stop_rule, double red_factor, double res_norm_min)
+// restart: beta = ||b - A x|| from its partial sums, stopping test on it, s = (beta, 0, ...), j = 0;
+// one block per instance.  V_0 is divided by beta by the start of the next cycle (A_SCALE0).
+__global__ void __launch_bounds__(kNT) b_restart(BTab t, BCtl *__restrict__ ctl, const double *__restrict__ partial,
+                                                 int stop_rule, double red_factor, double res_norm_min)
 {
   CD_PDL_ENTRY();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < t.K; k += gridDim.x * blockDim.x)
+  __shared__ double n2;
+  for (int k = blockIdx.x; k < t.K; k += gridDim.x)
   {
     BCtl &c = ctl[t.item[k]];
     if (!(c.state == ST_RUN && c.action == A_START)) continue;
-    const double beta = sqrt(c.nrm2);
+    __syncthreads();
+    b_gather(partial, t.total, t.bstart[k], t.bstart[k + 1], 1, &n2);
+    if (threadIdx.x != 0) continue;
+    const double beta = sqrt(n2);
     c.beta = beta;
     c.res = beta;
     if (c.its == 0 || stop_rule == 0) c.res0 = beta; // FgmresIte.C:557 (restart residual)
@@ -919,29 +1082,6 @@ __global__ void b_restart(BTab t, BCtl *__restrict__ ctl, int stop_rule, double 
     c.s[0] = beta;
     c.j = 0;
     c.action = A_SCALE0;
-  }
-}
-
-__global__ void b_scale0(BTab t, BCtl *__restrict__ ctl)
-{
-  CD_PDL_ENTRY();
-  for (int vb = blockIdx.x; vb < t.total; vb += gridDim.x)
-  {
-    const int k = find_item(t, vb), slot = t.item[k];
-    const BCtl &c = ctl[slot];
-    if (!(c.state == ST_RUN && c.action == A_SCALE0)) continue;
-    const int r = (vb - t.bstart[k]) * kVecRows + threadIdx.x;
-    if (r < c.n) c.V[r] /= c.beta;
-  }
-}
-
-__global__ void b_begin_step(BTab t, BCtl *__restrict__ ctl)
-{
-  CD_PDL_ENTRY();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < t.K; k += gridDim.x * blockDim.x)
-  {
-    BCtl &c = ctl[t.item[k]];
-    if (c.state == ST_RUN && c.action == A_SCALE0) c.action = A_STEP;
   }
 }
 
@@ -1275,6 +1415,8 @@ static int build_tables(cdgpu_ctx *ctx, Batch &b)
   auto all = [&](int, int) { return true; };
   fill(kVecRows, nrows, all, 0);
   add(b.fine_vec, v);
+  fill(kGsRows, nrows, all, 0);
+  add(b.fine_gs, v);
   fill(kCsrRows, nrows, all, 0);
   add(b.fine_csr, v);
   v.clear();
@@ -1347,8 +1489,8 @@ static int build_tables(cdgpu_ctx *ctx, Batch &b)
     pd.t->item = b.d_tab + pd.item_off;
     pd.t->bstart = b.d_tab + pd.bs_off;
   }
-  // partial sums: one slot block per virtual block of the largest table that writes them
-  size_t need = (size_t)std::max(b.fine_vec.total, b.fine_csr.total) * kSlots;
+  // partial sums: those of two Gram-Schmidt passes, or one per virtual block of the restart residual
+  const size_t need = std::max((size_t)2 * kSlots * b.fine_gs.total, (size_t)b.fine_csr.total);
   if (need > b.partial_cap)
   {
     if (b.d_partial) { cudaFree(b.d_partial); b.d_partial = nullptr; }
@@ -1386,6 +1528,8 @@ static int batch_cycle(cdgpu_ctx *ctx, Batch &b)
   };
   (void)cd_launch(b_mg_start, grid_of(ctx, b.fine_vec.total), kNT, 0, st, b.fine_vec, b.d_ctl, b.d_lev);
   CD_LAUNCHED(ctx);
+  // with Jacobi sweeps the last one of depth 0 leaves Z_j itself
+  const bool last_leaves_z = jac && post > 0;
   auto sweeps = [&](int d, int count, bool first_zero) -> int {
     const BTab &t = b.smooth[d];
     if (jac)
@@ -1395,8 +1539,13 @@ static int batch_cycle(cdgpu_ctx *ctx, Batch &b)
       {
         if (first_zero && s == 0)
         {
-          (void)cd_launch(b_jacobi_first, grid_of(ctx, t.total), kNT, 0, st, t, b.d_ctl, b.d_lev, d, src, omega);
-          CD_LAUNCHED(ctx);
+          // depth 0; below, the restriction has left the first sweep
+          if (d == 0)
+          {
+            (void)cd_launch(b_jacobi_first, grid_of(ctx, b.fine_vec.total), kNT, 0, st, b.fine_vec, b.d_ctl, b.d_lev,
+                            omega);
+            CD_LAUNCHED(ctx);
+          }
         }
         else if (int rc = rows(b_rows<BR_JACOBI>, t, d, src, 1 - src, omega))
           return rc;
@@ -1441,7 +1590,7 @@ static int batch_cycle(cdgpu_ctx *ctx, Batch &b)
     int rc = sweeps(d, pre, true);
     if (rc) return rc;
     if ((rc = rows(b_rows<BR_DEFECT>, b.smooth[d], d, after_pre, 0, 0.f))) return rc;
-    if ((rc = rows(b_rows<BR_RESTRICT>, b.restrict_[d], d, 0, 0, 0.f))) return rc;
+    if ((rc = rows(b_rows<BR_RESTRICT>, b.restrict_[d], d, 0, 0, jac && pre > 0 ? omega : 0.f))) return rc;
   }
   if (b.cta_smem > 0)
   {
@@ -1458,7 +1607,8 @@ static int batch_cycle(cdgpu_ctx *ctx, Batch &b)
       int src = after_pre;
       for (int s = 0; s < post; s++)
       {
-        if (int rc = rows(b_rows<BR_JACOBI>, b.smooth[d], d, src, 1 - src, omega)) return rc;
+        const int dst = last_leaves_z && d == 0 && s + 1 == post ? 2 : 1 - src;
+        if (int rc = rows(b_rows<BR_JACOBI>, b.smooth[d], d, src, dst, omega)) return rc;
         src = 1 - src;
       }
     }
@@ -1468,7 +1618,9 @@ static int batch_cycle(cdgpu_ctx *ctx, Batch &b)
       if (rc) return rc;
     }
   }
-  (void)cd_launch(b_mg_finish, grid_of(ctx, b.fine_vec.total), kNT, 0, st, b.fine_vec, b.d_ctl, b.d_lev, after_post);
+  // the other instances' result (with last_leaves_z only those of a single level)
+  (void)cd_launch(b_mg_finish, grid_of(ctx, b.fine_vec.total), kNT, 0, st, b.fine_vec, b.d_ctl, b.d_lev, after_post,
+                  last_leaves_z ? 1 : 0);
   CD_LAUNCHED(ctx);
   return CDGPU_OK;
 }
@@ -1478,30 +1630,27 @@ static int batch_iteration(cdgpu_ctx *ctx, Batch &b)
   const cdgpu_solver_params &p = b.p;
   cudaStream_t st = ctx->stream;
   const int gi = std::max(1, std::min((b.items.K + 127) / 128, ctx->sm_count * 4));
-  // restarts (and first starts): V_0 = b - A x, beta, V_0 /= beta
-  (void)cd_launch(b_matvec, grid_of(ctx, b.fine_csr.total), kNT, 0, st, b.fine_csr, b.d_ctl, 1, b.d_partial);
+  const BTab &gs = b.fine_gs;
+  double *p1 = b.d_partial, *p2 = p1 + (size_t)kSlots * gs.total;
+  const int gm = std::max(1, std::min(b.fine_csr.total, ctx->sm_count * 3)),
+            gg = std::max(1, std::min(gs.total, ctx->sm_count * 2));
+  // restarts (and first starts): V_0 = b - A x, beta (the cycle's start divides V_0 by it)
+  (void)cd_launch(b_matvec<true>, gm, kNT, 0, st, b.fine_csr, (const BCtl *)b.d_ctl, p1);
   CD_LAUNCHED(ctx);
-  (void)cd_launch(b_reduce, grid_of(ctx, b.fine_csr.K), kNT, 0, st, b.fine_csr, b.d_ctl, 2, 1, b.d_partial);
-  CD_LAUNCHED(ctx);
-  (void)cd_launch(b_restart, gi, 128, 0, st, b.items, b.d_ctl, p.stop_rule, p.red_factor, p.res_norm_min);
-  CD_LAUNCHED(ctx);
-  (void)cd_launch(b_scale0, grid_of(ctx, b.fine_vec.total), kNT, 0, st, b.fine_vec, b.d_ctl);
-  CD_LAUNCHED(ctx);
-  (void)cd_launch(b_begin_step, gi, 128, 0, st, b.items, b.d_ctl);
+  (void)cd_launch(b_restart, grid_of(ctx, b.fine_csr.K), kNT, 0, st, b.fine_csr, b.d_ctl, (const double *)p1, p.stop_rule,
+                  p.red_factor, p.res_norm_min);
   CD_LAUNCHED(ctx);
   // one Arnoldi step: z = M^{-1} v_j, w = A z, CGS2, Givens
   int rc = batch_cycle(ctx, b);
   if (rc) return rc;
-  (void)cd_launch(b_matvec, grid_of(ctx, b.fine_csr.total), kNT, 0, st, b.fine_csr, b.d_ctl, 0, b.d_partial);
+  (void)cd_launch(b_matvec<false>, gm, kNT, 0, st, b.fine_csr, (const BCtl *)b.d_ctl, p1);
   CD_LAUNCHED(ctx);
-  for (int mode = 0; mode < 3; mode++)
-  {
-    (void)cd_launch(b_gs, grid_of(ctx, b.fine_vec.total), kNT, 0, st, b.fine_vec, b.d_ctl, mode, b.d_partial);
-    CD_LAUNCHED(ctx);
-    (void)cd_launch(b_reduce, grid_of(ctx, b.fine_vec.K), kNT, 0, st, b.fine_vec, b.d_ctl, mode, 0, b.d_partial);
-    CD_LAUNCHED(ctx);
-  }
-  (void)cd_launch(b_givens, gi, 128, 0, st, b.items, b.d_ctl, p.maxit, p.minit, p.div_factor);
+  (void)cd_launch(b_gs<false>, gg, kNT, 0, st, gs, b.d_ctl, (const double *)nullptr, p1);
+  CD_LAUNCHED(ctx);
+  (void)cd_launch(b_gs<true>, gg, kNT, 0, st, gs, b.d_ctl, (const double *)p1, p2);
+  CD_LAUNCHED(ctx);
+  (void)cd_launch(b_givens, grid_of(ctx, gs.K), kNT, 0, st, gs, b.d_ctl, (const double *)p2, p.maxit, p.minit,
+                  p.div_factor);
   CD_LAUNCHED(ctx);
   (void)cd_launch(b_next_update, grid_of(ctx, b.fine_vec.total), kNT, 0, st, b.fine_vec, b.d_ctl);
   CD_LAUNCHED(ctx);

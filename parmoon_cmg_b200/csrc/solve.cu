@@ -28,6 +28,7 @@
 #include <type_traits>
 
 #include "internal.h"
+#include "warp.cuh"
 #include "csr.cuh"
 #include "mf.cuh"
 #include "mf64.cuh"
@@ -281,36 +282,6 @@ constexpr int kGsRowsInFlight = 16; // basis values a thread keeps in flight: ro
 
 // rows a thread takes at once, so that small K keeps as many loads in flight as large K
 template <int K> constexpr int gs_rows() { return K >= kGsRowsInFlight ? 1 : K >= 8 ? 2 : 4; }
-
-// Sums of N values over a warp: lane l returns the sum of v[l] (l < N), N <= 32.  At each of
-// the five steps a lane passes on the half of its values that the other lane keeps.
-template <int N> __device__ __forceinline__ double warp_sums(double (&v)[N])
-{
-  const int lane = threadIdx.x & 31;
-  int cnt = N;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-  {
-    const bool hi = lane & o;
-#pragma unroll
-    for (int j = 0; j < 16; j++)
-    {
-      if (j >= o || j >= cnt) continue;
-      if (j + o < cnt)
-      {
-        const double keep = hi ? v[j + o < N ? j + o : j] : v[j], give = hi ? v[j] : v[j + o < N ? j + o : j];
-        v[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-      }
-      else
-      {
-        const double other = __shfl_xor_sync(0xffffffffu, v[j], o);
-        v[j] = hi ? 0.0 : v[j] + other;
-      }
-    }
-    cnt = cnt < o ? cnt : o;
-  }
-  return v[0];
-}
 
 // a block's sums of acc[0..N) (and, with NORM, of sq in slot N) into partial[slot * stride +
 // block]; every thread of the block calls it
