@@ -24,7 +24,7 @@ int ensure_err_flag(cdgpu_ctx *ctx)
   if (rc) return rc;
   CD_CUDA(ctx, cudaMallocHost((void **)&ctx->h_err, sizeof(int)));
   *ctx->h_err = 0;
-  CD_CUDA(ctx, cudaMemset(ctx->d_err, 0, sizeof(int)));
+  CD_CUDA(ctx, cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
   return CDGPU_OK;
 }
 
@@ -195,8 +195,8 @@ int cdgpu_upload_space(cdgpu_ctx *ctx, int dim, int order, int n_cells, const do
     free_space(s);
     return rc;
   }
-  cudaError_t e = cudaMemcpy(s->d_coords, s->h_coords.data(), s->h_coords.size() * sizeof(double), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(s->d_gn, s->h_gn.data(), s->h_gn.size() * sizeof(int), cudaMemcpyHostToDevice);
+  cudaError_t e = upload(ctx, s->d_coords, s->h_coords.data(), s->h_coords.size() * sizeof(double));
+  if (e == cudaSuccess) e = upload(ctx, s->d_gn, s->h_gn.data(), s->h_gn.size() * sizeof(int));
   if (e != cudaSuccess) { free_space(s); return cuda_fail(ctx, e, "upload_space"); }
   // DOF -> cell incidence for the row-gather assembly
   std::vector<int> ptr, inc;
@@ -206,8 +206,8 @@ int cdgpu_upload_space(cdgpu_ctx *ctx, int dim, int order, int n_cells, const do
     free_space(s);
     return rc;
   }
-  e = cudaMemcpy(s->d_inc_ptr, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(s->d_inc, inc.data(), inc.size() * sizeof(int), cudaMemcpyHostToDevice);
+  e = upload(ctx, s->d_inc_ptr, ptr.data(), ptr.size() * sizeof(int));
+  if (e == cudaSuccess) e = upload(ctx, s->d_inc, inc.data(), inc.size() * sizeof(int));
   if (e != cudaSuccess) { free_space(s); return cuda_fail(ctx, e, "upload_space"); }
   ctx->spaces.push_back(s);
   *space_id = (int)ctx->spaces.size() - 1;
@@ -240,14 +240,14 @@ static int install_pattern(cdgpu_ctx *ctx, Space &s, int *d_kcol_built = nullptr
       (rc = dev_alloc(ctx, &s.d_dir_start, s.n_dof)) ||
       (rc = dev_alloc(ctx, &s.d_dir_rows, std::max<size_t>(1, dir_rows.size()))))
     return rc;
-  CD_CUDA(ctx, cudaMemcpy(s.d_row_ptr, s.h_row_ptr.data(), sizeof(int) * (s.n_dof + 1), cudaMemcpyHostToDevice));
+  CD_CUDA(ctx, upload(ctx, s.d_row_ptr, s.h_row_ptr.data(), sizeof(int) * (s.n_dof + 1)));
   if (!d_kcol_built)
-    CD_CUDA(ctx, cudaMemcpy(s.d_kcol, s.h_kcol.data(), sizeof(int) * s.nnz, cudaMemcpyHostToDevice));
-  CD_CUDA(ctx, cudaMemcpy(s.d_dir_start, dir_start.data(), sizeof(int) * s.n_dof, cudaMemcpyHostToDevice));
+    CD_CUDA(ctx, upload(ctx, s.d_kcol, s.h_kcol.data(), sizeof(int) * s.nnz));
+  CD_CUDA(ctx, upload(ctx, s.d_dir_start, dir_start.data(), sizeof(int) * s.n_dof));
   if (!dir_rows.empty())
-    CD_CUDA(ctx, cudaMemcpy(s.d_dir_rows, dir_rows.data(), sizeof(int) * dir_rows.size(), cudaMemcpyHostToDevice));
-  CD_CUDA(ctx, cudaMemset(s.d_row_ptr + s.n_dof + 1, 0, sizeof(int) * kCsrPad));
-  CD_CUDA(ctx, cudaMemset(s.d_kcol + s.nnz, 0, sizeof(int) * kCsrPad));
+    CD_CUDA(ctx, upload(ctx, s.d_dir_rows, dir_rows.data(), sizeof(int) * dir_rows.size()));
+  CD_CUDA(ctx, cudaMemsetAsync(s.d_row_ptr + s.n_dof + 1, 0, sizeof(int) * kCsrPad, ctx->stream));
+  CD_CUDA(ctx, cudaMemsetAsync(s.d_kcol + s.nnz, 0, sizeof(int) * kCsrPad, ctx->stream));
   s.shape = csr_shape(s.h_row_ptr.data(), s.n_dof);
   if ((rc = build_csr_tiles(ctx, s))) return rc;
   // a new pattern invalidates values sized for the old one and the slot map
@@ -360,7 +360,7 @@ int cdgpu_set_coeffs(cdgpu_ctx *ctx, int space_id, const cdgpu_coeffs *co, const
       if (!std::isfinite(h_table[i])) return fail(ctx, CDGPU_ERR_INVALID, "set_coeffs: non-finite table entry");
     int rc = dev_alloc(ctx, &s->d_tab, n);
     if (rc) return rc;
-    CD_CUDA(ctx, cudaMemcpy(s->d_tab, h_table, n * sizeof(double), cudaMemcpyHostToDevice));
+    CD_CUDA(ctx, upload(ctx, s->d_tab, h_table, n * sizeof(double)));
   }
   s->co_set = true;
   return CDGPU_OK;
@@ -717,14 +717,14 @@ int cdgpu_hierarchy(cdgpu_ctx *ctx, int n_levels, const int *space_ids, const in
       free_mg(h);
       return rc;
     }
-    cudaMemcpy(L.d_p_row, row.data(), row.size() * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(L.d_p_col, col.data(), col.size() * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(L.d_p_val, val.data(), val.size() * sizeof(double), cudaMemcpyHostToDevice);
-    cudaMemcpy(L.d_p_val32, val32.data(), val32.size() * sizeof(float), cudaMemcpyHostToDevice);
-    cudaMemcpy(L.d_r_row, rrow.data(), rrow.size() * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(L.d_r_col, rcol.data(), rcol.size() * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(L.d_r_val, rval.data(), rval.size() * sizeof(double), cudaMemcpyHostToDevice);
-    cudaError_t e = cudaMemcpy(L.d_r_val32, rval32.data(), rval32.size() * sizeof(float), cudaMemcpyHostToDevice);
+    upload(ctx, L.d_p_row, row.data(), row.size() * sizeof(int));
+    upload(ctx, L.d_p_col, col.data(), col.size() * sizeof(int));
+    upload(ctx, L.d_p_val, val.data(), val.size() * sizeof(double));
+    upload(ctx, L.d_p_val32, val32.data(), val32.size() * sizeof(float));
+    upload(ctx, L.d_r_row, rrow.data(), rrow.size() * sizeof(int));
+    upload(ctx, L.d_r_col, rcol.data(), rcol.size() * sizeof(int));
+    upload(ctx, L.d_r_val, rval.data(), rval.size() * sizeof(double));
+    cudaError_t e = upload(ctx, L.d_r_val32, rval32.data(), rval32.size() * sizeof(float));
     if (e != cudaSuccess) { free_mg(h); return cuda_fail(ctx, e, "hierarchy"); }
     L.p_shape = csr_shape(row.data(), f.n_dof);
     L.r_shape = csr_shape(rrow.data(), c.n_dof);

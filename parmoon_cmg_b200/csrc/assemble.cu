@@ -774,7 +774,7 @@ static int ensure_quadtab(cdgpu_ctx *ctx, Space &s)
   packed.resize(packed.size() + 2, 0.0);
   int rc = dev_alloc(ctx, &s.d_quadtab, packed.size());
   if (rc) return rc;
-  CD_CUDA(ctx, cudaMemcpy(s.d_quadtab, packed.data(), packed.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CD_CUDA(ctx, upload(ctx, s.d_quadtab, packed.data(), packed.size() * sizeof(double)));
   return CDGPU_OK;
 }
 
@@ -1038,7 +1038,7 @@ int assemble_space(cdgpu_ctx *ctx, Space &s, int disctype, const double *h_dir, 
       std::vector<double> both(R);
       both.insert(both.end(), r.begin(), r.end());
       if ((rc = dev_alloc(ctx, &s.d_ref, both.size()))) return rc;
-      CD_CUDA(ctx, cudaMemcpy(s.d_ref, both.data(), both.size() * sizeof(double), cudaMemcpyHostToDevice));
+      CD_CUDA(ctx, upload(ctx, s.d_ref, both.data(), both.size() * sizeof(double)));
       s.ref_disctype = disctype;
     }
     if (!s.d_cellcoef && (rc = dev_alloc(ctx, &s.d_cellcoef, (size_t)s.n_cells * (CD_MAXT + 4))))

@@ -1286,7 +1286,7 @@ static int ensure_colors(cdgpu_ctx *ctx, Hierarchy &h)
     rows.insert(rows.end(), L.h_color_ptr.begin(), L.h_color_ptr.end());
     int rc = dev_alloc(ctx, &L.d_color_rows, rows.size());
     if (rc) return rc;
-    CD_CUDA(ctx, cudaMemcpy(L.d_color_rows, rows.data(), sizeof(int) * rows.size(), cudaMemcpyHostToDevice));
+    CD_CUDA(ctx, upload(ctx, L.d_color_rows, rows.data(), sizeof(int) * rows.size()));
     L.n_colors = nc;
   }
   return CDGPU_OK;
@@ -1343,14 +1343,14 @@ static int grow(cdgpu_ctx *ctx, Batch &b, int need)
       (rc = dev_alloc(ctx, &st, cap)))
     return rc;
   CD_CUDA(ctx, cudaMallocHost((void **)&hst, sizeof(int) * cap));
-  CD_CUDA(ctx, cudaMemset(ctl, 0, sizeof(BCtl) * cap));
-  CD_CUDA(ctx, cudaMemset(lev, 0, sizeof(BLevel) * cap * kMaxDepth));
-  CD_CUDA(ctx, cudaMemset(st, 0, sizeof(int) * cap));
+  CD_CUDA(ctx, cudaMemsetAsync(ctl, 0, sizeof(BCtl) * cap, ctx->stream));
+  CD_CUDA(ctx, cudaMemsetAsync(lev, 0, sizeof(BLevel) * cap * kMaxDepth, ctx->stream));
+  CD_CUDA(ctx, cudaMemsetAsync(st, 0, sizeof(int) * cap, ctx->stream));
   if (b.cap)
   {
-    CD_CUDA(ctx, cudaMemcpy(ctl, b.d_ctl, sizeof(BCtl) * b.cap, cudaMemcpyDeviceToDevice));
-    CD_CUDA(ctx, cudaMemcpy(lev, b.d_lev, sizeof(BLevel) * b.cap * kMaxDepth, cudaMemcpyDeviceToDevice));
-    CD_CUDA(ctx, cudaMemcpy(st, b.d_state, sizeof(int) * b.cap, cudaMemcpyDeviceToDevice));
+    CD_CUDA(ctx, cudaMemcpyAsync(ctl, b.d_ctl, sizeof(BCtl) * b.cap, cudaMemcpyDeviceToDevice, ctx->stream));
+    CD_CUDA(ctx, cudaMemcpyAsync(lev, b.d_lev, sizeof(BLevel) * b.cap * kMaxDepth, cudaMemcpyDeviceToDevice, ctx->stream));
+    CD_CUDA(ctx, cudaMemcpyAsync(st, b.d_state, sizeof(int) * b.cap, cudaMemcpyDeviceToDevice, ctx->stream));
     cudaFree(b.d_ctl);
     cudaFree(b.d_lev);
     cudaFree(b.d_state);
@@ -2040,7 +2040,8 @@ int cdgpu_batch_tcd_step(cdgpu_ctx *ctx, int batch_id, int iterations, int *max_
     if (b.tcd_looped)
     {
       int left = 0;
-      CD_CUDA(ctx, cudaMemcpy(&left, b.d_loop, sizeof(int), cudaMemcpyDeviceToHost));
+      CD_CUDA(ctx, cudaMemcpyAsync(&left, b.d_loop, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+      CD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
       *max_iterations = (budget - std::max(0, left)) + extra;
     }
     else

@@ -303,6 +303,15 @@ template <typename T> int dev_alloc(cdgpu_ctx *ctx, T **p, size_t n)
   return CDGPU_OK;
 }
 
+// Host array to device memory, ordered before everything enqueued on ctx->stream afterwards; the
+// source may be reused on return.  (A plain cudaMemcpy from pageable memory runs on the legacy
+// stream, with which the context's non-blocking streams do not synchronise, and may return while
+// the last staged piece is still on its way; cudaMemset does not wait at all.)
+inline cudaError_t upload(const cdgpu_ctx *ctx, void *dst, const void *src, size_t bytes)
+{
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
+}
+
 // host-side setup algorithms (setup.cpp)
 void build_pattern(const Space &s, std::vector<int> &row_ptr, std::vector<int> &kcol);
 void build_incidence(const Space &s, std::vector<int> &ptr, std::vector<int> &inc);

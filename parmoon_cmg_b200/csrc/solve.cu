@@ -1215,7 +1215,7 @@ int build_csr_tiles(cdgpu_ctx *ctx, Space &s)
   int rc;
   if ((rc = ensure_err_flag(ctx))) return rc;
   if ((rc = dev_alloc(ctx, &s.d_tiles, tiles.size()))) return rc;
-  CD_CUDA(ctx, cudaMemcpy(s.d_tiles, tiles.data(), sizeof(int2) * tiles.size(), cudaMemcpyHostToDevice));
+  CD_CUDA(ctx, upload(ctx, s.d_tiles, tiles.data(), sizeof(int2) * tiles.size()));
   if (tma_ctas_per_sm(0) <= 0) return cuda_fail(ctx, cudaErrorInvalidConfiguration, "TMA product: no resident CTA");
   s.n_tiles = (int)tiles.size() - 1;
   return CDGPU_OK;
@@ -1251,7 +1251,7 @@ static int tune_tma(cdgpu_ctx *ctx, Space &s)
     if (ctas <= 0 || !make_tiles(s, kTmaVariants[v].cap, tma_rows(v), tiles)) continue;
     int2 *dt = nullptr;
     if ((rc = dev_alloc(ctx, &dt, tiles.size()))) break;
-    CD_CUDA(ctx, cudaMemcpy(dt, tiles.data(), sizeof(int2) * tiles.size(), cudaMemcpyHostToDevice));
+    CD_CUDA(ctx, upload(ctx, dt, tiles.data(), sizeof(int2) * tiles.size()));
     const int nt = (int)tiles.size() - 1;
     const int grid = std::max(1, std::min(nt, ctx->sm_count * ctas));
     CsrArgs<double> p = csr_args<double>(s, x);
@@ -1319,8 +1319,8 @@ template <typename T> static int alloc_vecs(cdgpu_ctx *ctx, LevelVec<T> &v, int 
   if ((rc = dev_alloc(ctx, &v.sol, n)) || (rc = dev_alloc(ctx, &v.alt, n)) ||
       (rc = dev_alloc(ctx, &v.rhs, n)) || (rc = dev_alloc(ctx, &v.def, n)))
     return rc;
-  CD_CUDA(ctx, cudaMemset(v.sol, 0, sizeof(T) * n));
-  CD_CUDA(ctx, cudaMemset(v.alt, 0, sizeof(T) * n));
+  CD_CUDA(ctx, cudaMemsetAsync(v.sol, 0, sizeof(T) * n, ctx->stream));
+  CD_CUDA(ctx, cudaMemsetAsync(v.alt, 0, sizeof(T) * n, ctx->stream));
   return CDGPU_OK;
 }
 
