@@ -225,12 +225,21 @@ __global__ void __launch_bounds__(256, MINB) csr_pipe_kernel(CsrArgs<T> p)
   }
 }
 
-// grid of a CSR launch: one pass over the rows, at most 8 blocks of 256 threads per SM
-inline int csr_grid(const cdgpu_ctx *ctx, const CsrShape &sh, int rows)
+// Blocks of 256 threads per SM of the CSR kernels: the bound under which they are compiled (32
+// registers in FP32, 48 in FP64; without one the compiler took 64 and 89, and half the warps fit)
+// and the limit of their grids, so that every block of a large matrix is resident and takes the
+// same share of the rows.  Whole solves, unbounded kernels in grids of 8 blocks per SM against
+// this: CD2D Q2 192^2 mixed 3,720 -> 3,400 us, CD3D Q1 48^3 mixed 1,730 -> 1,600, one TCD2D Q2
+// 128^2 step in FP64 1,430 -> 1,300 (6 blocks FP32: 3,457 us on the first; 4 FP64: within 1 % of 5).
+// Rows of 33-128 entries (8 threads each, 16 loads in flight) keep 4 blocks: 5 and 6 were slower.
+template <typename T> constexpr int csr_blocks(int gs) { return gs == 8 ? 4 : sizeof(T) == 8 ? 5 : 8; }
+
+// grid of a CSR launch: one pass over the rows, at most the resident blocks
+template <typename T> inline int csr_grid(const cdgpu_ctx *ctx, const CsrShape &sh, int rows)
 {
   const long per_block = 256 / sh.gs;
   const long need = (rows + per_block - 1) / per_block;
-  return (int)std::max<long>(1, std::min<long>(need, (long)ctx->sm_count * 8));
+  return (int)std::max<long>(1, std::min<long>(need, (long)ctx->sm_count * csr_blocks<T>(sh.gs)));
 }
 
 template <typename T, int MODE>
@@ -238,22 +247,20 @@ inline void launch_csr(cdgpu_ctx *ctx, const CsrShape &sh, const CsrArgs<T> &pa,
 {
   CsrArgs<T> p = pa;
   p.pre = ctx->pdl_pre ? 1 : 0;
+  constexpr int B1 = csr_blocks<T>(1), B2 = csr_blocks<T>(2), B4 = csr_blocks<T>(4), B8 = csr_blocks<T>(8),
+                B32 = csr_blocks<T>(32);
   switch (sh.gs)
   {
-    case 1: (void)cd_launch(csr_kernel<T, 1, 8, MODE>, grid, 256, 0, ctx->stream, p); break;
-    case 2: (void)cd_launch(csr_kernel<T, 2, 8, MODE>, grid, 256, 0, ctx->stream, p); break;
-    case 4: (void)cd_launch(csr_kernel<T, 4, 8, MODE>, grid, 256, 0, ctx->stream, p); break;
+    case 1: (void)cd_launch(csr_kernel<T, 1, 8, MODE, B1>, grid, 256, 0, ctx->stream, p); break;
+    case 2: (void)cd_launch(csr_kernel<T, 2, 8, MODE, B2>, grid, 256, 0, ctx->stream, p); break;
+    case 4: (void)cd_launch(csr_kernel<T, 4, 8, MODE, B4>, grid, 256, 0, ctx->stream, p); break;
     case 8:
-      // FP64: at most 64 registers, so that 4 CTAs (32 warps) share an SM instead of 3; the
-      // 32^3 Q2 product went from 73 to 54 us with a cold L2
       if (sizeof(T) == 4 && (MODE == CM_JACOBI || MODE == CM_DEFECT))
-        (void)cd_launch(csr_pipe_kernel<T, 8, 8, MODE>, grid, 256, 0, ctx->stream, p);
-      else if (sizeof(T) == 8)
-        (void)cd_launch(csr_kernel<T, 8, 16, MODE, 4>, grid, 256, 0, ctx->stream, p);
+        (void)cd_launch(csr_pipe_kernel<T, 8, 8, MODE, B8>, grid, 256, 0, ctx->stream, p);
       else
-        (void)cd_launch(csr_kernel<T, 8, 16, MODE>, grid, 256, 0, ctx->stream, p);
+        (void)cd_launch(csr_kernel<T, 8, 16, MODE, B8>, grid, 256, 0, ctx->stream, p);
       break;
-    default: (void)cd_launch(csr_kernel<T, 32, 8, MODE>, grid, 256, 0, ctx->stream, p); break;
+    default: (void)cd_launch(csr_kernel<T, 32, 8, MODE, B32>, grid, 256, 0, ctx->stream, p); break;
   }
 }
 

@@ -794,7 +794,7 @@ template <typename T> static void csr_jacobi(cdgpu_ctx *ctx, const Space &s, con
   p.y = xo;
   p.omega = omega;
   if (launch_tma<T, CM_JACOBI>(ctx, s, p, tma_grid(ctx, s))) return;
-  launch_csr<T, CM_JACOBI>(ctx, s.shape, p, csr_grid(ctx, s.shape, s.n_dof));
+  launch_csr<T, CM_JACOBI>(ctx, s.shape, p, csr_grid<T>(ctx, s.shape, s.n_dof));
 }
 // grid: the launch's number of blocks (and of partial sums), from defect_grid
 template <typename T>
@@ -810,14 +810,14 @@ static void csr_defect(cdgpu_ctx *ctx, const Space &s, const T *x, const T *f, T
 template <typename T> static int defect_grid(const cdgpu_ctx *ctx, const Space &s)
 {
   if (std::is_same<T, double>::value && s.n_tiles > 0 && ctx->d_err) return tma_grid(ctx, s);
-  return csr_grid(ctx, s.shape, s.n_dof);
+  return csr_grid<T>(ctx, s.shape, s.n_dof);
 }
 template <typename T> static void csr_spmv(cdgpu_ctx *ctx, const Space &s, const T *x, T *y)
 {
   CsrArgs<T> p = csr_args<T>(s, x);
   p.y = y;
   if (launch_tma<T, CM_SPMV>(ctx, s, p, tma_grid(ctx, s))) return;
-  launch_csr<T, CM_SPMV>(ctx, s.shape, p, csr_grid(ctx, s.shape, s.n_dof));
+  launch_csr<T, CM_SPMV>(ctx, s.shape, p, csr_grid<T>(ctx, s.shape, s.n_dof));
 }
 // coarse rhs = R d (zero on non-active coarse rows), coarse solution reset
 template <typename T>
@@ -832,7 +832,7 @@ static void csr_restrict(cdgpu_ctx *ctx, const Level &L, const Space &sc, const 
   p.x = d;
   p.y = crhs;
   p.y2 = csol;
-  launch_csr<T, CM_RESTRICT>(ctx, L.r_shape, p, csr_grid(ctx, L.r_shape, p.n));
+  launch_csr<T, CM_RESTRICT>(ctx, L.r_shape, p, csr_grid<T>(ctx, L.r_shape, p.n));
 }
 // sol += damp * P xc on active fine rows
 template <typename T>
@@ -847,7 +847,7 @@ static void csr_prolong(cdgpu_ctx *ctx, const Level &L, const Space &s, const T 
   p.x = xc;
   p.y = sol;
   p.omega = damp;
-  launch_csr<T, CM_PROLONG>(ctx, L.p_shape, p, csr_grid(ctx, L.p_shape, p.n_active));
+  launch_csr<T, CM_PROLONG>(ctx, L.p_shape, p, csr_grid<T>(ctx, L.p_shape, p.n_active));
 }
 
 // the matrix-free FP64 operator (mf64.cuh) applies to Q2 hexahedra assembled by the affine
