@@ -24,6 +24,7 @@ template <typename T> struct CsrArgs
   T *y = nullptr, *y2 = nullptr;
   T omega = 0;
   double *partial = nullptr;
+  double *const *io = nullptr; // Jacobi: (in, out) slot of the captured cycle whose result this is
   // 1: the kernel loads its first rows' pointers, columns and values before waiting for its
   // predecessor (set for the kernels of the captured multigrid cycle, where no kernel writes
   // a matrix; see CD_PDL_WAIT)
@@ -53,17 +54,21 @@ __device__ __forceinline__ void csr_epilogue(const CsrArgs<T> &p, int r, T s, do
   {
     // x + omega D^{-1} (f - A x) = (1 - omega) x + omega (f - sum_{j != r} a_rj x_j) / a_rr
     // (MGLevel3D.C:443-537, MGLevel2D.C:318-368); Dirichlet rows take the right-hand side
-    if (r < p.n_active)
-      p.y[r] = p.x[r] + p.omega * (p.f[r] - s) / p.diag[r];
+    const T v = r < p.n_active ? p.x[r] + p.omega * (p.f[r] - s) / p.diag[r] : p.f[r];
+    // the last sweep of the finest level leaves the cycle's result in FP64 (the graph's slot)
+    if (p.io)
+      p.io[1][r] = (double)v;
     else
-      p.y[r] = p.f[r];
+      p.y[r] = v;
   }
   else if (MODE == CM_RESTRICT)
   {
-    // coarse rhs = R d on active rows, zero elsewhere (CorrectDefect, MGLevel3D.C:588);
-    // coarse solution reset (MGLevel3D.C:557)
-    p.y[r] = r < p.n_active ? s : T(0);
-    p.y2[r] = T(0);
+    // coarse rhs = R d on active rows, zero elsewhere (CorrectDefect, MGLevel3D.C:588); coarse
+    // solution reset (MGLevel3D.C:557), or with a diagonal already its first damped Jacobi sweep
+    // from zero, omega f / d (the Dirichlet columns carry zeros)
+    const T f = r < p.n_active ? s : T(0);
+    p.y[r] = f;
+    p.y2[r] = p.diag && r < p.n_active ? p.omega * f / p.diag[r] : T(0);
   }
   else // CM_PROLONG: sol += damp * (P xc) on active fine rows (Update, MGLevel3D.C:539)
   {

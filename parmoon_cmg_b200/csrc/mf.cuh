@@ -443,11 +443,21 @@ static_assert(mf_tc_smem_bytes<13>() <= kMfTcSmem && mf_tc_smem_bytes<10>() <= k
 
 enum { MF_JACOBI = 0, MF_DEFECT = 1, MF_SPMV = 2 };
 
+// a row's result; with io (the last sweep of a cycle) into the cycle's FP64 output vector
+__device__ __forceinline__ void mf_put(float *out, double *const *io, int r, float v)
+{
+  if (io)
+    io[1][r] = (double)v;
+  else
+    out[r] = v;
+}
+
 template <int NBF, int MODE>
 __global__ void mf_row_kernel(int n, int na, int n_cells, const int *__restrict__ inc_ptr,
                               const int *__restrict__ inc, const float *__restrict__ ybuf,
                               const float *__restrict__ x, const float *__restrict__ f,
-                              const float *__restrict__ diag, float *__restrict__ out, float omega, int pre)
+                              const float *__restrict__ diag, float *__restrict__ out, float omega, int pre,
+                              double *const *__restrict__ io)
 {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
@@ -466,7 +476,7 @@ __global__ void mf_row_kernel(int n, int na, int n_cells, const int *__restrict_
   if (r >= na)
   {
     // Dirichlet rows are identity rows
-    out[r] = MODE == MF_JACOBI ? f[r] : MODE == MF_DEFECT ? f[r] - x[r] : x[r];
+    mf_put(out, io, r, MODE == MF_JACOBI ? f[r] : MODE == MF_DEFECT ? f[r] - x[r] : x[r]);
     return;
   }
   if (!pre) load_inc();
@@ -486,7 +496,7 @@ __global__ void mf_row_kernel(int n, int na, int n_cells, const int *__restrict_
     const int K = inc[t] / NBF, li = inc[t] - K * NBF;
     s += ybuf[(size_t)li * n_cells + K];
   }
-  out[r] = MODE == MF_JACOBI ? x[r] + omega * (f[r] - s) / diag[r] : MODE == MF_DEFECT ? f[r] - s : s;
+  mf_put(out, io, r, MODE == MF_JACOBI ? x[r] + omega * (f[r] - s) / diag[r] : MODE == MF_DEFECT ? f[r] - s : s);
 }
 
 // The DOF -> (cell, local index) incidence of every active row as up to 8 indices into the
@@ -518,7 +528,8 @@ __global__ void mf_inc8_kernel(int n_active, int nbf, int n_cells, const int *__
 template <int MODE>
 __global__ void mf_row8_kernel(int n, int na, const int *__restrict__ inc8, const float *__restrict__ ybuf,
                                const float *__restrict__ x, const float *__restrict__ f,
-                               const float *__restrict__ diag, float *__restrict__ out, float omega, int pre)
+                               const float *__restrict__ diag, float *__restrict__ out, float omega, int pre,
+                              double *const *__restrict__ io)
 {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
@@ -532,7 +543,7 @@ __global__ void mf_row8_kernel(int n, int na, const int *__restrict__ inc8, cons
   if (r >= na)
   {
     // Dirichlet rows are identity rows
-    out[r] = MODE == MF_JACOBI ? f[r] : MODE == MF_DEFECT ? f[r] - x[r] : x[r];
+    mf_put(out, io, r, MODE == MF_JACOBI ? f[r] : MODE == MF_DEFECT ? f[r] - x[r] : x[r]);
     return;
   }
   if (!pre)
@@ -548,7 +559,7 @@ __global__ void mf_row8_kernel(int n, int na, const int *__restrict__ inc8, cons
 #pragma unroll
   for (int j = 0; j < 8; j++)
     if (ix[j] >= 0) s += yv[j];
-  out[r] = MODE == MF_JACOBI ? x[r] + omega * (f[r] - s) / diag[r] : MODE == MF_DEFECT ? f[r] - s : s;
+  mf_put(out, io, r, MODE == MF_JACOBI ? x[r] + omega * (f[r] - s) / diag[r] : MODE == MF_DEFECT ? f[r] - s : s);
 }
 
 // FP32 copies of the cell coefficients (first T of each cell's T + Tr) and of the tensors
@@ -625,20 +636,20 @@ inline void mf_apply_cells(cdgpu_ctx *ctx, const Space &s, const float *x, bool 
 
 template <int MODE>
 inline void mf_rows(cdgpu_ctx *ctx, const Space &s, const float *x, const float *f, const float *diag, float *out,
-                    float omega)
+                    float omega, double *const *io = nullptr)
 {
   const int grid = (s.n_dof + 255) / 256;
   if (s.d_inc8)
   {
     (void)cd_launch(mf_row8_kernel<MODE>, grid, 256, 0, ctx->stream, s.n_dof, s.n_active, (const int *)s.d_inc8,
-                    (const float *)s.d_ybuf, x, f, diag, out, omega, ctx->pdl_pre ? 1 : 0);
+                    (const float *)s.d_ybuf, x, f, diag, out, omega, ctx->pdl_pre ? 1 : 0, io);
     return;
   }
   switch (s.nbf)
   {
-    case 27: (void)cd_launch(mf_row_kernel<27, MODE>, grid, 256, 0, ctx->stream, s.n_dof, s.n_active, s.n_cells, s.d_inc_ptr, s.d_inc, s.d_ybuf, x, f, diag, out, omega, ctx->pdl_pre ? 1 : 0); break;
-    case 9: (void)cd_launch(mf_row_kernel<9, MODE>, grid, 256, 0, ctx->stream, s.n_dof, s.n_active, s.n_cells, s.d_inc_ptr, s.d_inc, s.d_ybuf, x, f, diag, out, omega, ctx->pdl_pre ? 1 : 0); break;
-    case 8: (void)cd_launch(mf_row_kernel<8, MODE>, grid, 256, 0, ctx->stream, s.n_dof, s.n_active, s.n_cells, s.d_inc_ptr, s.d_inc, s.d_ybuf, x, f, diag, out, omega, ctx->pdl_pre ? 1 : 0); break;
-    default: (void)cd_launch(mf_row_kernel<4, MODE>, grid, 256, 0, ctx->stream, s.n_dof, s.n_active, s.n_cells, s.d_inc_ptr, s.d_inc, s.d_ybuf, x, f, diag, out, omega, ctx->pdl_pre ? 1 : 0); break;
+    case 27: (void)cd_launch(mf_row_kernel<27, MODE>, grid, 256, 0, ctx->stream, s.n_dof, s.n_active, s.n_cells, s.d_inc_ptr, s.d_inc, s.d_ybuf, x, f, diag, out, omega, ctx->pdl_pre ? 1 : 0, io); break;
+    case 9: (void)cd_launch(mf_row_kernel<9, MODE>, grid, 256, 0, ctx->stream, s.n_dof, s.n_active, s.n_cells, s.d_inc_ptr, s.d_inc, s.d_ybuf, x, f, diag, out, omega, ctx->pdl_pre ? 1 : 0, io); break;
+    case 8: (void)cd_launch(mf_row_kernel<8, MODE>, grid, 256, 0, ctx->stream, s.n_dof, s.n_active, s.n_cells, s.d_inc_ptr, s.d_inc, s.d_ybuf, x, f, diag, out, omega, ctx->pdl_pre ? 1 : 0, io); break;
+    default: (void)cd_launch(mf_row_kernel<4, MODE>, grid, 256, 0, ctx->stream, s.n_dof, s.n_active, s.n_cells, s.d_inc_ptr, s.d_inc, s.d_ybuf, x, f, diag, out, omega, ctx->pdl_pre ? 1 : 0, io); break;
   }
 }

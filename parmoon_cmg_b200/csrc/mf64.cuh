@@ -226,10 +226,12 @@ __global__ void __launch_bounds__(256) mf64_row_kernel(int n, int na, int n_cell
                                                        const int *__restrict__ inc, const int *__restrict__ inc8,
                                                        const double *__restrict__ ybuf,
                                                        const double *__restrict__ x, const double *__restrict__ f,
-                                                       double *__restrict__ out, double *__restrict__ partial,
-                                                       const double *__restrict__ diag, double omega)
+                                                       double *out, double *__restrict__ partial,
+                                                       const double *__restrict__ diag, double omega,
+                                                       double *const *__restrict__ io)
 {
   CD_PDL_ENTRY();
+  if (MODE == MF64_JACOBI && io) out = io[1]; // the last sweep of a cycle leaves its result
   double acc = 0;
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
   {

@@ -786,13 +786,15 @@ template <typename T, int MODE> static bool launch_tma(cdgpu_ctx *ctx, const Spa
   }
   return false;
 }
-template <typename T> static void csr_jacobi(cdgpu_ctx *ctx, const Space &s, const T *x, const T *f, T *xo, T omega)
+template <typename T>
+static void csr_jacobi(cdgpu_ctx *ctx, const Space &s, const T *x, const T *f, T *xo, T omega, double *const *io)
 {
   CsrArgs<T> p = csr_args<T>(s, x);
   p.f = f;
   p.diag = dg<T>(s);
   p.y = xo;
   p.omega = omega;
+  p.io = io;
   if (launch_tma<T, CM_JACOBI>(ctx, s, p, tma_grid(ctx, s))) return;
   launch_csr<T, CM_JACOBI>(ctx, s.shape, p, csr_grid<T>(ctx, s.shape, s.n_dof));
 }
@@ -819,9 +821,10 @@ template <typename T> static void csr_spmv(cdgpu_ctx *ctx, const Space &s, const
   if (launch_tma<T, CM_SPMV>(ctx, s, p, tma_grid(ctx, s))) return;
   launch_csr<T, CM_SPMV>(ctx, s.shape, p, csr_grid<T>(ctx, s.shape, s.n_dof));
 }
-// coarse rhs = R d (zero on non-active coarse rows), coarse solution reset
+// coarse rhs = R d (zero on non-active coarse rows); coarse solution reset, or (first) its first
+// Jacobi sweep from zero
 template <typename T>
-static void csr_restrict(cdgpu_ctx *ctx, const Level &L, const Space &sc, const T *d, T *crhs, T *csol)
+static void csr_restrict(cdgpu_ctx *ctx, const Level &L, const Space &sc, const T *d, T *crhs, T *csol, bool first, T omega)
 {
   CsrArgs<T> p;
   p.n = sc.n_dof;
@@ -832,6 +835,11 @@ static void csr_restrict(cdgpu_ctx *ctx, const Level &L, const Space &sc, const 
   p.x = d;
   p.y = crhs;
   p.y2 = csol;
+  if (first)
+  {
+    p.diag = dg<T>(sc);
+    p.omega = omega;
+  }
   launch_csr<T, CM_RESTRICT>(ctx, L.r_shape, p, csr_grid<T>(ctx, L.r_shape, p.n));
 }
 // sol += damp * P xc on active fine rows
@@ -922,14 +930,15 @@ static int mf64_rows_grid(const cdgpu_ctx *ctx, const Space &s)
 }
 template <int MODE>
 static void mf64_rows(cdgpu_ctx *ctx, const Space &s, const double *x, const double *f, double *out, double *partial,
-                      const double *diag = nullptr, double omega = 0)
+                      const double *diag = nullptr, double omega = 0, double *const *io = nullptr)
 {
   (void)cd_launch(mf64_row_kernel<MODE>, mf64_rows_grid(ctx, s), 256, 0, ctx->stream, s.n_dof, s.n_active,
                   s.n_cells, (const int *)s.d_inc_ptr, (const int *)s.d_inc, (const int *)s.d_inc8,
-                  (const double *)s.d_ybuf64, x, f, out, partial, diag, omega);
+                  (const double *)s.d_ybuf64, x, f, out, partial, diag, omega, io);
 }
 
-template <typename T> static int jacobi_sweep(cdgpu_ctx *ctx, Level &L, T omega)
+// one sweep; with io (the last one of a cycle) its result goes to the cycle's output vector
+template <typename T> static int jacobi_sweep(cdgpu_ctx *ctx, Level &L, T omega, double *const *io = nullptr)
 {
   LevelVec<T> &v = vecs<T>(L);
   const Space &s = *L.sp;
@@ -939,7 +948,7 @@ template <typename T> static int jacobi_sweep(cdgpu_ctx *ctx, Level &L, T omega)
     {
       mf_apply_cells(ctx, s, v.sol);
       CD_LAUNCHED(ctx);
-      mf_rows<MF_JACOBI>(ctx, s, v.sol, v.rhs, s.d_diag32, v.alt, omega);
+      mf_rows<MF_JACOBI>(ctx, s, v.sol, v.rhs, s.d_diag32, v.alt, omega, io);
       CD_LAUNCHED(ctx);
       std::swap(v.sol, v.alt);
       return CDGPU_OK;
@@ -949,12 +958,12 @@ template <typename T> static int jacobi_sweep(cdgpu_ctx *ctx, Level &L, T omega)
   {
     mf64_cells(ctx, s, v.sol);
     CD_LAUNCHED(ctx);
-    mf64_rows<MF64_JACOBI>(ctx, s, v.sol, v.rhs, v.alt, nullptr, s.d_diag, omega);
+    mf64_rows<MF64_JACOBI>(ctx, s, v.sol, v.rhs, v.alt, nullptr, s.d_diag, omega, io);
     CD_LAUNCHED(ctx);
     std::swap(v.sol, v.alt);
     return CDGPU_OK;
   }
-  csr_jacobi<T>(ctx, s, v.sol, v.rhs, v.alt, omega);
+  csr_jacobi<T>(ctx, s, v.sol, v.rhs, v.alt, omega, io);
   CD_LAUNCHED(ctx);
   std::swap(v.sol, v.alt);
   return CDGPU_OK;
@@ -984,7 +993,9 @@ struct CycleState
   bool active_zero[64];
 };
 
-template <typename T> static int smooth(cdgpu_ctx *ctx, Hierarchy &h, CycleState &cs, int i, int count)
+// io: the last of these sweeps is the last of the whole cycle
+template <typename T>
+static int smooth(cdgpu_ctx *ctx, Hierarchy &h, CycleState &cs, int i, int count, double *const *io = nullptr)
 {
   Level &L = h.lev[i];
   T omega = (T)cs.p->omega;
@@ -994,7 +1005,7 @@ template <typename T> static int smooth(cdgpu_ctx *ctx, Hierarchy &h, CycleState
     if (cs.active_zero[i])
       rc = jacobi_first<T>(ctx, L, omega, cs.sol_zero[i] ? 1 : 0);
     else
-      rc = jacobi_sweep<T>(ctx, L, omega);
+      rc = jacobi_sweep<T>(ctx, L, omega, k + 1 == count ? io : nullptr);
     if (rc) return rc;
     cs.active_zero[i] = cs.sol_zero[i] = false;
   }
@@ -1066,9 +1077,13 @@ template <typename T> static int cycle(cdgpu_ctx *ctx, Hierarchy &h, CycleState 
   }
   if (!done) csr_defect<T>(ctx, s, v.sol, v.rhs, v.def, nullptr, defect_grid<T>(ctx, s));
   CD_LAUNCHED(ctx);
-  csr_restrict<T>(ctx, L, sc, v.def, vc.rhs, vc.sol);
+  // the level below starts from zero: its first pre-smoothing sweep is left by the restriction
+  // (not where the level is solved or applied as a whole)
+  const bool first = i - 1 > 0 && i - 1 != h.dense_level && cs.p->pre > 0;
+  csr_restrict<T>(ctx, L, sc, v.def, vc.rhs, vc.sol, first, (T)cs.p->omega);
   CD_LAUNCHED(ctx);
-  cs.sol_zero[i - 1] = cs.active_zero[i - 1] = true;
+  cs.sol_zero[i - 1] = cs.active_zero[i - 1] = !first;
+  cs.pre_done[i - 1] = first ? 1 : 0;
   for (int j = 0; j < cs.rec[i]; j++)
     if ((rc = cycle<T>(ctx, h, cs, i - 1))) return rc;
   if (cs.p->cycle < 1) cs.rec[i] = 1;
@@ -1076,7 +1091,8 @@ template <typename T> static int cycle(cdgpu_ctx *ctx, Hierarchy &h, CycleState 
   CD_LAUNCHED(ctx);
   // the corrected iterate is not zero, also where no pre-smoothing sweep has cleared the flags
   cs.sol_zero[i] = cs.active_zero[i] = false;
-  return smooth<T>(ctx, h, cs, i, cs.p->post);
+  // the finest level's last sweep writes the cycle's result itself
+  return smooth<T>(ctx, h, cs, i, cs.p->post, i + 1 == (int)h.lev.size() ? h.d_io : nullptr);
 }
 
 // enqueue one preconditioner application z = M^{-1} r (TMultiGridScaIte::Iterate with zero
@@ -1121,6 +1137,7 @@ template <typename T> static int mg_record(cdgpu_ctx *ctx, Hierarchy &h, const c
   }
   int rc = cycle<T>(ctx, h, cs, L - 1);
   if (rc) return rc;
+  if (L > 1 && p.post > 0) return CDGPU_OK; // left by the last sweep
   (void)cd_launch(mg_finish_kernel<T>, (n + 255) / 256, 256, 0, ctx->stream, n, v.sol, h.d_io);
   CD_LAUNCHED(ctx);
   return CDGPU_OK;
