@@ -50,25 +50,6 @@ template <int GS, typename T> __device__ __forceinline__ T group_sum(T v)
   return v;
 }
 
-// first sweep when the active part of x is zero: only Dirichlet columns (numbered last,
-// so at the end of every sorted row, from dir_start[r]) can contribute
-template <typename T>
-__global__ void jacobi_first_kernel(int n, int n_active, const int *__restrict__ rp,
-                                    const int *__restrict__ kc, const int *__restrict__ dir_start,
-                                    const T *__restrict__ a, const T *__restrict__ diag,
-                                    const T *__restrict__ x, const T *__restrict__ f,
-                                    T *__restrict__ xo, T omega, int x_all_zero)
-{
-  CD_PDL_ENTRY();
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  if (r >= n_active) { xo[r] = f[r]; return; }
-  T s = f[r];
-  if (!x_all_zero)
-    for (int j = dir_start[r]; j < rp[r + 1]; j++) s -= a[j] * x[kc[j]];
-  xo[r] = omega * s / diag[r];
-}
-
 // start of a cycle on the finest level fused with its first damped-Jacobi sweep: the
 // right-hand side is the (FP64) input vector read through the pointer slot io[0]; the start
 // vector is zero on active rows and the right-hand side on Dirichlet rows
@@ -969,18 +950,6 @@ template <typename T> static int jacobi_sweep(cdgpu_ctx *ctx, Level &L, T omega,
   return CDGPU_OK;
 }
 
-template <typename T> static int jacobi_first(cdgpu_ctx *ctx, Level &L, T omega, int all_zero)
-{
-  LevelVec<T> &v = vecs<T>(L);
-  const Space &s = *L.sp;
-  (void)cd_launch(jacobi_first_kernel<T>, (s.n_dof + 255) / 256, 256, 0, ctx->stream, 
-      s.n_dof, s.n_active, s.d_row_ptr, s.d_kcol, s.d_dir_start, mat<T>(s), dg<T>(s), v.sol, v.rhs,
-      v.alt, omega, all_zero);
-  CD_LAUNCHED(ctx);
-  std::swap(v.sol, v.alt);
-  return CDGPU_OK;
-}
-
 // ---------------------------------------------------------------------------
 // V/W/F cycle
 // ---------------------------------------------------------------------------
@@ -988,9 +957,7 @@ struct CycleState
 {
   const cdgpu_solver_params *p;
   int rec[64];
-  int pre_done[64];    // pre-smoothing sweeps already done (fused into the cycle's start)
-  bool sol_zero[64];   // active part and Dirichlet part zero
-  bool active_zero[64];
+  int pre_done[64]; // pre-smoothing sweeps left by the kernel that set the level's start vector
 };
 
 // io: the last of these sweeps is the last of the whole cycle
@@ -1001,14 +968,7 @@ static int smooth(cdgpu_ctx *ctx, Hierarchy &h, CycleState &cs, int i, int count
   T omega = (T)cs.p->omega;
   int rc;
   for (int k = 0; k < count; k++)
-  {
-    if (cs.active_zero[i])
-      rc = jacobi_first<T>(ctx, L, omega, cs.sol_zero[i] ? 1 : 0);
-    else
-      rc = jacobi_sweep<T>(ctx, L, omega, k + 1 == count ? io : nullptr);
-    if (rc) return rc;
-    cs.active_zero[i] = cs.sol_zero[i] = false;
-  }
+    if ((rc = jacobi_sweep<T>(ctx, L, omega, k + 1 == count ? io : nullptr))) return rc;
   return CDGPU_OK;
 }
 
@@ -1033,7 +993,6 @@ template <typename T> static int coarse_solve(cdgpu_ctx *ctx, Hierarchy &h, Cycl
                                                          cs.p->coarse_red);
     CD_LAUNCHED(ctx);
   }
-  cs.sol_zero[0] = cs.active_zero[0] = false;
   return CDGPU_OK;
 }
 
@@ -1047,7 +1006,6 @@ template <typename T> static int cycle(cdgpu_ctx *ctx, Hierarchy &h, CycleState 
     (void)cd_launch(dense_cycle_kernel<T>, std::max(1, (na + 7) / 8), 256, 0, ctx->stream, na, (const double *)h.d_dense,
                     (const T *)v.rhs, v.sol, ctx->pdl_pre ? 1 : 0);
     CD_LAUNCHED(ctx);
-    cs.sol_zero[i] = cs.active_zero[i] = false;
     return CDGPU_OK;
   }
   if (i == 0) return coarse_solve<T>(ctx, h, cs);
@@ -1082,15 +1040,12 @@ template <typename T> static int cycle(cdgpu_ctx *ctx, Hierarchy &h, CycleState 
   const bool first = i - 1 > 0 && i - 1 != h.dense_level && cs.p->pre > 0;
   csr_restrict<T>(ctx, L, sc, v.def, vc.rhs, vc.sol, first, (T)cs.p->omega);
   CD_LAUNCHED(ctx);
-  cs.sol_zero[i - 1] = cs.active_zero[i - 1] = !first;
   cs.pre_done[i - 1] = first ? 1 : 0;
   for (int j = 0; j < cs.rec[i]; j++)
     if ((rc = cycle<T>(ctx, h, cs, i - 1))) return rc;
   if (cs.p->cycle < 1) cs.rec[i] = 1;
   csr_prolong<T>(ctx, L, s, vc.sol, v.sol, (T)cs.p->gmg_damp);
   CD_LAUNCHED(ctx);
-  // the corrected iterate is not zero, also where no pre-smoothing sweep has cleared the flags
-  cs.sol_zero[i] = cs.active_zero[i] = false;
   // the finest level's last sweep writes the cycle's result itself
   return smooth<T>(ctx, h, cs, i, cs.p->post, i + 1 == (int)h.lev.size() ? h.d_io : nullptr);
 }
@@ -1111,11 +1066,7 @@ template <typename T> static int mg_record(cdgpu_ctx *ctx, Hierarchy &h, const c
   // SetRecursion(levels = L-1), MultiGrid3D.C:691-703
   cs.rec[1] = 1;
   for (int k = 2; k <= L - 1; k++) cs.rec[k] = p.cycle > 0 ? p.cycle : 2;
-  for (int k = 0; k < L; k++)
-  {
-    cs.sol_zero[k] = cs.active_zero[k] = false;
-    cs.pre_done[k] = 0;
-  }
+  for (int k = 0; k < L; k++) cs.pre_done[k] = 0;
   if (L > 1 && p.pre >= 1)
   {
     // zero start and the first pre-smoothing sweep of the finest level in one kernel
@@ -1133,7 +1084,6 @@ template <typename T> static int mg_record(cdgpu_ctx *ctx, Hierarchy &h, const c
   {
     (void)cd_launch(mg_start_kernel<T>, (n + 255) / 256, 256, 0, ctx->stream, n, F.sp->n_active, h.d_io, v.rhs, v.sol);
     CD_LAUNCHED(ctx);
-    cs.active_zero[L - 1] = true;
   }
   int rc = cycle<T>(ctx, h, cs, L - 1);
   if (rc) return rc;
