@@ -9,7 +9,9 @@
 //   M <- M + (tau*theta2 + tau*theta1)*A     (the system matrix)
 //   solve M u = B
 //   M <- M - tau*theta1*A                    (RestoreMassMat)
-// so the rounding of every step is the reference's.
+// so the rounding of every update is the reference's; all of it but the solve is one pass over
+// the entries (tcd_system_kernel).
+#include <algorithm>
 #include <cmath>
 
 #include "internal.h"
@@ -38,34 +40,96 @@ void free_tcd(Tcd *t)
   delete t;
 }
 
-// y += alpha * x over the entries of the active rows [0, n_active_entries)
-__global__ void matadd_kernel(long n, double alpha, const double *__restrict__ x, double *__restrict__ y)
-{
-  CD_PDL_ENTRY();
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) y[i] += alpha * x[i];
-}
+// One step's matrix work on every level, and the finest right-hand side, in one pass over the
+// entries (8 lanes per row, so the entries of a warp's rows are read and written as whole
+// lines; up to four entries per lane in flight).  Entry by entry, with M read once:
+//   m  = M - tau theta2 A           (where the level takes this update)
+//   s += m x                        (finest level: the row's share of B)
+//   m += c A                        (the system matrix: FP64, FP32 and diagonal copies)
+//   M <- m - tau theta1 A           (what RestoreMassMat leaves; the solve reads the copies)
+// each update rounded as the separate passes of MatAdd round it.  Dirichlet rows keep M and
+// take B = f; their x = f comes in a launch of its own, the active rows read the old x.
+// Bound by DRAM/L2 bytes (40 per entry) on large levels and by launches on small ones:
+// 128^2 Q2 cells on 7 levels, a step's matrix work took 24 launches (a MatAdd before, in and
+// after the solve and an install kernel per level, one thread per row in the latter):
+// 155 us, now 2 launches, 17 us.
+constexpr int kTcdLevels = 32; // levels of one launch (the argument's size stays below 4 KB)
+constexpr int kTcdRows = 32;   // rows of a block
 
-// B = tau*th3*f_old + tau*th4*f + (M x) on active rows; B = f and x = f on Dirichlet rows
-__global__ void tcd_rhs_kernel(int n, int n_active, const int *__restrict__ rp, const int *__restrict__ kc,
-                               const double *__restrict__ M, const double *__restrict__ f_old,
-                               const double *__restrict__ f, double c3, double c4, double *__restrict__ x,
-                               double *__restrict__ B)
+struct TcdLevel
+{
+  const int *rp, *kc;
+  const double *A;
+  double *M, *a, *diag;
+  float *a32, *diag32;
+  double c; // of the second update
+  int n, n_active, block0, half;
+};
+
+struct TcdArgs
+{
+  int levels, fine; // fine: lev[0] is the finest level
+  double c_half, c_restore, c3, c4;
+  const double *f_old, *f, *x;
+  double *B;
+  TcdLevel lev[kTcdLevels];
+};
+
+__global__ void __launch_bounds__(256) tcd_system_kernel(const __grid_constant__ TcdArgs p)
 {
   CD_PDL_ENTRY();
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  if (r >= n_active)
-  {
-    B[r] = f[r];
-    return;
-  }
+  constexpr int U = 4;
+  int k = 0;
+  while (k + 1 < p.levels && (int)blockIdx.x >= p.lev[k + 1].block0) k++;
+  const TcdLevel &l = p.lev[k];
+  const int lane = threadIdx.x % 8, r = ((int)blockIdx.x - l.block0) * kTcdRows + threadIdx.x / 8;
+  const bool valid = r < l.n, active = r < l.n_active, rhs = p.fine && k == 0 && active;
+  const int j1 = valid ? l.rp[r + 1] : 0;
   double s = 0;
-  for (int j = rp[r]; j < rp[r + 1]; j++) s += M[j] * x[kc[j]];
+  for (int j0 = valid ? l.rp[r] + lane : 0; j0 < j1; j0 += 8 * U)
+  {
+    double m[U], a[U], x[U];
+    int col[U];
+#pragma unroll
+    for (int q = 0; q < U; q++)
+    {
+      const int j = j0 + 8 * q;
+      const bool in = j < j1;
+      col[q] = in ? l.kc[j] : -1;
+      m[q] = in ? l.M[j] : 0.0;
+      a[q] = in && active ? l.A[j] : 0.0;
+    }
+    if (rhs)
+#pragma unroll
+      for (int q = 0; q < U; q++) x[q] = col[q] >= 0 ? p.x[col[q]] : 0.0;
+#pragma unroll
+    for (int q = 0; q < U; q++)
+    {
+      const int j = j0 + 8 * q;
+      if (j >= j1) break;
+      double v = m[q];
+      if (active)
+      {
+        if (l.half) v += p.c_half * a[q];
+        if (rhs) s += v * x[q];
+        v += l.c * a[q];
+        double back = v;
+        back += p.c_restore * a[q];
+        l.M[j] = back;
+      }
+      l.a[j] = v;
+      l.a32[j] = (float)v;
+      if (col[q] == r) { l.diag[r] = v; l.diag32[r] = (float)v; }
+    }
+  }
+  if (!p.fine || k != 0) return; // block-uniform
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, 8);
+  if (lane != 0 || !valid) return;
   double b = 0.0;
-  b += c3 * f_old[r];
-  b += c4 * f[r];
-  B[r] = b + s;
+  b += p.c3 * p.f_old[r];
+  b += p.c4 * p.f[r];
+  p.B[r] = active ? b + s : p.f[r];
 }
 
 __global__ void dirichlet_copy_kernel(int n, int n_active, const double *__restrict__ f, double *__restrict__ x)
@@ -73,32 +137,6 @@ __global__ void dirichlet_copy_kernel(int n, int n_active, const double *__restr
   CD_PDL_ENTRY();
   int r = n_active + blockIdx.x * blockDim.x + threadIdx.x;
   if (r < n) x[r] = f[r];
-}
-
-// system matrix of a level into the space's value arrays (f64, f32 copy, diagonals)
-__global__ void install_system_kernel(int n, const int *__restrict__ rp, const int *__restrict__ kc,
-                                      const double *__restrict__ M, double *__restrict__ a, float *__restrict__ a32,
-                                      double *__restrict__ diag, float *__restrict__ diag32)
-{
-  CD_PDL_ENTRY();
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  for (int j = rp[r]; j < rp[r + 1]; j++)
-  {
-    double v = M[j];
-    a[j] = v;
-    a32[j] = (float)v;
-    if (kc[j] == r) { diag[r] = v; diag32[r] = (float)v; }
-  }
-}
-
-static int matadd(cdgpu_ctx *ctx, const Space &s, double alpha, const double *x, double *y)
-{
-  long n = s.h_row_ptr[s.n_active];
-  if (n == 0) return CDGPU_OK;
-  (void)cd_launch(matadd_kernel, (unsigned)((n + 255) / 256), 256, 0, ctx->stream, n, alpha, x, y);
-  CD_LAUNCHED(ctx);
-  return CDGPU_OK;
 }
 
 static Tcd *get_tcd(cdgpu_ctx *ctx, int id)
@@ -111,7 +149,8 @@ static Tcd *get_tcd(cdgpu_ctx *ctx, int id)
 // side goes to rhs_dst
 static int assemble_into(cdgpu_ctx *ctx, Tcd &t, int disctype, std::vector<double *> &dst, double *rhs_dst)
 {
-  for (size_t l = 0; l < t.h->lev.size(); l++)
+  // finest level first: while it runs, the launches of the small levels are queued behind it
+  for (size_t l = t.h->lev.size(); l-- > 0;)
   {
     Space &s = *t.h->lev[l].sp;
     const bool fine = l + 1 == t.h->lev.size();
@@ -209,45 +248,48 @@ int cdgpu_tcd_step_device(cdgpu_ctx *ctx, int tcd_id, const cdgpu_solver_params 
   cudaSetDevice(ctx->device);
   Hierarchy &h = *t->h;
   const int L = (int)h.lev.size();
-  int rc;
   const Space &f = *h.lev[L - 1].sp;
   // 2D (SystemTCD2D.C): M <- M - tau theta2 A on every level, so that the coarse levels get
   // the finest level's sequence of updates; 3D (SystemTCD3D.C:257-278): on the finest level
   // only, the coarser levels' system matrices are M + tau theta1 A
   const bool fine_only = f.dim == 3;
-  for (int l = 0; l < L; l++)
-    if (!(fine_only && l < L - 1) && (rc = matadd(ctx, *h.lev[l].sp, -tau * theta2, t->A[l], t->M[l]))) return rc;
-  (void)cd_launch(tcd_rhs_kernel, (f.n_dof + 255) / 256, 256, 0, ctx->stream, f.n_dof, f.n_active, f.d_row_ptr, f.d_kcol,
-                                                                t->M[L - 1], t->d_f_old, t->d_f, tau * theta3,
-                                                                tau * theta4, d_sol, t->d_B);
-  CD_LAUNCHED(ctx);
+  // finest level first, in the blocks of one launch
+  for (int top = L - 1; top >= 0;)
+  {
+    TcdArgs a;
+    a.levels = 0;
+    a.fine = top == L - 1;
+    a.c_half = -tau * theta2;
+    a.c_restore = -tau * theta1;
+    a.c3 = tau * theta3;
+    a.c4 = tau * theta4;
+    a.f_old = t->d_f_old;
+    a.f = t->d_f;
+    a.x = d_sol;
+    a.B = t->d_B;
+    long blocks = 0;
+    for (; top >= 0 && a.levels < kTcdLevels; top--)
+    {
+      Space &s = *h.lev[top].sp;
+      const bool half = !(fine_only && top < L - 1);
+      const double c = half ? -a.c_half + tau * theta1 : tau * theta1;
+      a.lev[a.levels++] = {s.d_row_ptr, s.d_kcol, t->A[top], t->M[top], s.d_a, s.d_diag, s.d_a32, s.d_diag32, c,
+                           s.n_dof, s.n_active, (int)blocks, half ? 1 : 0};
+      blocks += (s.n_dof + kTcdRows - 1) / kTcdRows;
+      s.mf_T = 0; // the system matrix is a combination, not one affine assembly
+      s.assembly_version++;
+    }
+    (void)cd_launch(tcd_system_kernel, (unsigned)std::max(1L, blocks), 256, 0, ctx->stream, a);
+    CD_LAUNCHED(ctx);
+  }
   if (f.n_dof > f.n_active)
   {
     (void)cd_launch(dirichlet_copy_kernel, (f.n_dof - f.n_active + 255) / 256, 256, 0, ctx->stream, f.n_dof, f.n_active, t->d_f,
                                                                                      d_sol);
     CD_LAUNCHED(ctx);
   }
-  const double gamma = -tau * theta2;
-  for (int l = 0; l < L; l++)
-  {
-    Space &s = *h.lev[l].sp;
-    const double c = fine_only && l < L - 1 ? tau * theta1 : -gamma + tau * theta1;
-    if ((rc = matadd(ctx, s, c, t->A[l], t->M[l]))) return rc;
-    s.mf_T = 0; // the system matrix is a combination, not one affine assembly
-    (void)cd_launch(install_system_kernel, (s.n_dof + 255) / 256, 256, 0, ctx->stream, s.n_dof, s.d_row_ptr, s.d_kcol, t->M[l],
-                                                                        s.d_a, s.d_a32, s.d_diag, s.d_diag32);
-    CD_LAUNCHED(ctx);
-    s.assembly_version++;
-  }
   cdgpu_solve_info local{};
-  rc = run_solve(ctx, h, *p, t->d_B, d_sol, info ? info : &local);
-  // RestoreMassMat: M <- M - tau theta1 A, whatever the solve returned
-  for (int l = 0; l < L; l++)
-  {
-    int r2 = matadd(ctx, *h.lev[l].sp, -tau * theta1, t->A[l], t->M[l]);
-    if (!rc) rc = r2;
-  }
-  return rc;
+  return run_solve(ctx, h, *p, t->d_B, d_sol, info ? info : &local);
 }
 
 int cdgpu_tcd_step(cdgpu_ctx *ctx, int tcd_id, const cdgpu_solver_params *p, double tau, double theta1,
