@@ -375,10 +375,13 @@ class TSystemTCD2D:
     def Step(self, sol, tau, theta1, theta2, theta3, theta4, params=None):
         params = params or solver_params()
         info = SolveInfo()
-        x = _f64(sol).copy()
+        # the library reads the old solution from and writes the new one into ``sol`` where it can
+        in_place = _is_f64_out(sol, self.N_DOF)
+        x = sol if in_place else _f64(sol).copy()
         self.ctx.check(self.ctx.lib.cdgpu_tcd_step(self.ctx.h, self.tcd, C.byref(params), tau, theta1,
                                                    theta2, theta3, theta4, _p(x), C.byref(info)))
-        sol[:] = x
+        if not in_place:
+            sol[:] = x
         return info
 
 
