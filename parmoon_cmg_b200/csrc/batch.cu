@@ -355,16 +355,23 @@ template <int OP> __global__ void __launch_bounds__(kNT, kRowBlocks) b_rows(cons
     const int n = OP == BR_RESTRICT ? L.nc : OP == BR_PROLONG ? L.na : OP == BR_COLOR ? __ldg(p.cstart + p.t.K + k) : L.n;
     const int na = OP == BR_RESTRICT ? L.nca : OP == BR_JACOBI ? L.na : n; // rows with a sum
     const int *list = OP == BR_COLOR ? L.color_rows + __ldg(p.cstart + k) : nullptr;
+    constexpr bool kSweep = OP == BR_JACOBI || OP == BR_COLOR;
+    const bool scale = kSweep || (OP == BR_RESTRICT && p.omega != 0.f); // the result is divided by the diagonal
+    const float *dg = OP == BR_RESTRICT ? C.d32 : L.d32, *f = L.rhs;
+    float *y = OP == BR_RESTRICT ? C.rhs : OP == BR_DEFECT ? L.def : OP == BR_COLOR ? L.v[0] : L.v[p.dst & 1];
+    float *y0 = OP == BR_RESTRICT ? C.v[p.omega != 0.f ? 1 : 0] : nullptr;
+    const float *own = OP == BR_JACOBI ? x : y; // the vector an update adds to
     const int i1 = min(n, (ve - b0) * kCsrRows);
     int i = (vb - b0) * kCsrRows + sub, r = 0, b = 0, e = 0, c[U];
-    float v[U];
-    auto fetch = [&]() {
+    float v[U], xc[U], d = 1.f, fr = 0.f, xr = 0.f;
+    auto fetch = [&]() { // what no kernel of the cycle writes
       r = OP == BR_COLOR ? (i < i1 ? __ldg(list + i) : 0) : i;
       b = e = 0;
       if (i < i1 && (OP == BR_COLOR || i < na))
       {
         b = __ldg(rp + r);
         e = __ldg(rp + r + 1);
+        if (scale) d = __ldg(dg + r);
       }
 #pragma unroll
       for (int u = 0; u < U; u++)
@@ -374,51 +381,64 @@ template <int OP> __global__ void __launch_bounds__(kNT, kRowBlocks) b_rows(cons
         v[u] = j < e ? __ldg(a + j) : 0.f;
       }
     };
+    auto gather = [&]() { // the vectors
+#pragma unroll
+      for (int u = 0; u < U; u++) xc[u] = c[u] >= 0 ? x[c[u]] : 0.f;
+      if (i < i1)
+      {
+        if (kSweep || OP == BR_DEFECT) fr = f[r];
+        if (kSweep || OP == BR_PROLONG) xr = own[r];
+      }
+    };
     fetch();
     if (!waited)
     {
       CD_PDL_WAIT();
       waited = true;
     }
+    gather(); // together with the instance's state
     const BCtl &ctl = p.ctl[slot];
-    double *Z = OP == BR_JACOBI && p.dst == 2 ? ctl.Z + (size_t)ctl.j * ctl.n : nullptr;
     if (stepping(ctl))
+    {
+      double *Z = OP == BR_JACOBI && p.dst == 2 ? ctl.Z + (size_t)ctl.j * ctl.n : nullptr;
       for (int base = (vb - b0) * kCsrRows; base < i1; base += kCsrRows)
       {
         const bool ok = i < i1;
         const int row = r;
         float s = 0;
 #pragma unroll
-        for (int u = 0; u < U; u++)
-          if (c[u] >= 0) s += v[u] * x[c[u]];
+        for (int u = 0; u < U; u++) s += v[u] * xc[u];
         for (int j = b + lane + 4 * U; j < e; j += 4) s += a[j] * x[kc[j]];
+        const float dr = d, rr = fr, o = xr;
         i += kCsrRows;
-        if (base + kCsrRows < i1) fetch();
+        if (base + kCsrRows < i1)
+        {
+          fetch();
+          gather();
+        }
         s = bsum<4>(s);
         if (!ok || lane != 0) continue;
         if (OP == BR_JACOBI)
         {
-          const float y = row < na ? x[row] + p.omega * (L.rhs[row] - s) / L.d32[row] : L.rhs[row];
+          const float z = row < na ? o + p.omega * (rr - s) / dr : rr;
           if (p.dst == 2)
-            Z[row] = (double)y;
+            Z[row] = (double)z;
           else
-            L.v[p.dst][row] = y;
+            y[row] = z;
         }
         else if (OP == BR_COLOR)
-          L.v[0][row] += p.omega * (L.rhs[row] - s) / L.d32[row];
+          y[row] = o + p.omega * (rr - s) / dr;
         else if (OP == BR_DEFECT)
-          L.def[row] = L.rhs[row] - s;
+          y[row] = rr - s;
         else if (OP == BR_RESTRICT)
         {
-          C.rhs[row] = row < na ? s : 0.f;
-          if (p.omega == 0.f)
-            C.v[0][row] = 0.f;
-          else
-            C.v[1][row] = row < na ? p.omega * s / C.d32[row] : 0.f;
+          y[row] = row < na ? s : 0.f;
+          y0[row] = p.omega != 0.f && row < na ? p.omega * s / dr : 0.f;
         }
         else
-          L.v[p.dst][row] += p.omega * s;
+          y[row] = o + p.omega * s;
       }
+    }
     vb = ve;
     k++;
   }
