@@ -206,7 +206,7 @@ int cdgpu_defect(cdgpu_ctx *ctx, int space_id, const double *h_x, const double *
 int cdgpu_spmv_device(cdgpu_ctx *ctx, int space_id, const double *d_x, double *d_y);
 /* The FP64 product, defect and Jacobi sweep of a matrix larger than L2 stream its tiles into
  * shared memory with bulk copies; the tile shape (nonzeros per tile, pipeline stages, CTAs
- * per SM) is chosen by timing every variant on the matrix at the first solve that uses it.
+ * per SM) is chosen by timing every variant on the matrix at its first FP64 solve.
  * This copies a one-line report of that choice (or "not tuned yet") into buf.  No reference
  * counterpart (MatVect / Defect, src/FE/Blas2.C:11-99, are the operations). */
 int cdgpu_product_tuning(cdgpu_ctx *ctx, int space_id, char *buf, int len);

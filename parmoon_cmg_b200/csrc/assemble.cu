@@ -5,15 +5,15 @@
 // src/FE/Matrix.C:111, src/FE/Structure.C:98; src/System/AssembleMat3D.C:765-787).
 // Here the matrix is assembled row by row instead: a group of threads owns one
 // CSR row, walks the cells containing the row's DOF in ascending cell order (the
-// same order in which the reference's cell loop adds into that row), finds each
-// column's slot by binary search in the row's own column list held in shared
-// memory, and accumulates in shared memory.  Every entry is written exactly once
+// same order in which the reference's cell loop adds into that row), takes each
+// column's slot from a map made once per pattern (binary search in the row's column
+// list), and accumulates in shared memory.  Every entry is written exactly once
 // with coalesced stores, there are no atomics and no colouring, and the sum order
 // per entry is the reference's.  Local values come from one of two producers:
 //   * affine fast path: for parallelogram / parallelepiped cells with constant
 //     coefficients the local matrix is sum_t coef[cell][t] * R_t over reference
 //     tensors R_t (see reference_tensors in setup.cpp); coef is computed per cell
-//     (cell_coef_kernel) and the row kernel evaluates local entries on the fly;
+//     (cell_coef_kernel), the local matrices formed from it (affine_local_kernel) and gathered;
 //   * quadrature path: local matrices by Gauss quadrature of the reference's
 //     per-point forms (quad.cuh), stored and then gathered.
 #include <climits>

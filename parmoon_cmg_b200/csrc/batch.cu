@@ -1,12 +1,14 @@
 // Batched GMG-FGMRES: many independent convection-diffusion solves advanced together.
 //
 // Every kernel of an FGMRES iteration is one grouped launch over all running instances: a
-// launch gets a table of (instance slot, first virtual block) pairs, and each virtual
-// block finds its instance by binary search and works on a fixed row range of that
-// instance's level.  Blocks loop over virtual blocks (grid <= 8 blocks per SM), so one
-// launch covers any number of instances of any sizes.  The FGMRES control -- Gram-Schmidt
+// launch gets a table of (instance slot, first virtual block) pairs, a virtual block being
+// a fixed row range of the instance's level.  In the row and vector kernels of the cycle a
+// block takes a contiguous range of virtual blocks and looks up its first instance only;
+// in the others each virtual block finds its instance by binary search.  One launch covers
+// any number of instances of any sizes; the coarse levels of an instance (b_cta_cycle) and
+// its Givens and restart work take one block each.  The FGMRES control -- Gram-Schmidt
 // coefficients, Givens rotations, stopping and divergence tests, restarts -- lives in a
-// per-instance device control block (BCtl) and is updated by per-instance threads, so the
+// per-instance device control block (BCtl) and is updated by a block per instance, so the
 // host never waits on an instance: it launches iterations and polls a state array.
 //
 // Per instance the algorithm is the mixed form of cdgpu_solve: FGMRES(m) in FP64 on the
@@ -360,7 +362,12 @@ __device__ __forceinline__ float sor_update(float x, float r, float d, float ome
 
 // Blocks per SM (40 stationary instances with SSOR and 16 time-dependent ones with Jacobi, solve
 // phases included: 62.5 and 32.2 ms with 4, 66.9 and 31.7 with 5, 73.5 and 36.2 with 6, whose
-// registers leave fewer loads in flight).
+// registers leave fewer loads in flight).  Grids of 3 or 2 blocks per SM, which leave room for the
+// next launch's blocks beside these, are no faster: 44.7 and 27.1 ms with 4, 44.8 and 29.6 with 3,
+// 47.3 and 34.7 with 2.  A launch is a chain of dependent loads (2-4 us at 64 rows per block and
+// fewer than one wave): what no kernel of the cycle writes is read before the wait, every vector
+// entry together with the instance's state after it (48.0 and 28.4 ms with the loads one after
+// the other).
 constexpr int kRowBlocks = 4;
 template <int OP> __global__ void __launch_bounds__(kNT, kRowBlocks) b_rows(const __grid_constant__ BRowArgs p)
 {
@@ -512,8 +519,8 @@ __global__ void b_coarse(BTab t, const BCtl *__restrict__ ctl, const BLevel *__r
 // The cycle of an instance's coarse levels, from depth cta_top (at most cta_rows active rows) to
 // the exact solve and back, by one block with the iterates and right-hand sides in shared memory:
 // f of depth cta_top in, v[out] of that depth out.  The sums are those of b_rows and b_coarse.
-// These levels are bound by the number of dependent steps: a multicolour SSOR V(2,2) takes 72
-// colour classes and more per level, 2.1 us each as a grouped launch and about 1 us as a barrier
+// These levels are bound by the number of dependent steps: a multicolour SSOR V(2,2) takes 66
+// colour classes and more per level, 2.1 us each as a grouped launch and 0.7 us as a barrier
 // of one block, whose matrices (up to some 900 rows) stay in its L1; damped Jacobi takes 7
 // launches per level.  40 stationary instances with SSOR, limit on the rows: none 62.5 ms, 256
 // 55.5, 1,024 50.8, 4,096 57.1; 16 time-dependent ones with Jacobi: none 32.2 ms, 256 31.5, 1,024

@@ -257,7 +257,9 @@ int cuda_fail(cdgpu_ctx *ctx, cudaError_t e, const char *what);
 // (griddepcontrol.wait) before it reads or writes anything the predecessor may touch, and
 // only then lets its own successor be scheduled (griddepcontrol.launch_dependents).  So at
 // most two kernels of a chain are resident at once, and the later one runs only the part
-// before its wait: the launch, the CTA scheduling and, in kernels of the captured multigrid
+// before its wait (the batch's row passes, many short launches in a row, let their successor in
+// at once: several may be resident, each still waiting for all before it, and what they read
+// before the wait is written by no kernel of the cycle): the launch, the CTA scheduling and, in kernels of the captured multigrid
 // cycle, loads of data that no kernel of the cycle writes (matrices, transfer operators,
 // incidence lists, reference tensors).  Without the launch attribute both instructions
 // return at once.

@@ -9,8 +9,9 @@
 // computes only to print residuals (before pre-smoothing, after the update, after
 // post-smoothing) change no state and are not computed.  Jacobi sweeps write into a
 // second buffer and swap pointers instead of copying sol into aux first
-// (MGLevel3D.C:455), which gives the same values.  A level whose solution is known
-// to be zero (after Reset) starts with a sweep that reads no matrix row.
+// (MGLevel3D.C:455), which gives the same values.  A level's first sweep from zero reads no
+// matrix row: the restriction (or the start of the cycle) leaves it with the right-hand side.
+// The coarsest levels of a V-cycle with the exact coarse solve are one dense product (coarse.cuh).
 //
 // FGMRES follows TFgmresIte::Iterate (src/FE/FgmresIte.C:236-582): same restart,
 // stopping and divergence rules, the same Givens rotations computed on the host in
@@ -1100,7 +1101,7 @@ static bool same_cycle_params(const cdgpu_solver_params &a, const cdgpu_solver_p
          a.coarse_red == b.coarse_red && a.omega == b.omega && a.gmg_damp == b.gmg_damp;
 }
 
-// The whole V/W/F cycle (about 7 kernels per level) is captured once into a CUDA graph
+// The whole V/W/F cycle (about 6 kernels per level) is captured once into a CUDA graph
 // and replayed for every basis vector; only the two pointers in h.d_io change.
 // io_ready: the kernel before this call already set the graph's (in, out) slot to (r, z)
 static int mg_apply(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, const double *r, double *z,
