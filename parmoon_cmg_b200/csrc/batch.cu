@@ -29,6 +29,7 @@
 
 #include "internal.h"
 #include "warp.cuh"
+#include "gj.cuh"
 
 namespace
 {
@@ -2379,7 +2380,12 @@ static int submit_impl(cdgpu_ctx *ctx, Batch &b, int mg_id, const cdgpu_coeffs *
       free_inst(ctx, in);
       return rc;
     }
-    if (na > 0)
+    if (na > 0 && na <= kGjWarpRows)
+    {
+      (void)cd_launch(gj_warp_kernel, 1, 32, 0, ctx->stream, na, c.d_row_ptr, c.d_dir_start, c.d_kcol, B.a64, cinv, flag);
+      CD_LAUNCHED(ctx);
+    }
+    else if (na > 0)
     {
       b_dense_active<<<na, 128, 0, ctx->stream>>>(na, c.d_row_ptr, c.d_kcol, B.a64, cinv);
       CD_LAUNCHED(ctx);

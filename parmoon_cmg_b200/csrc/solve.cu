@@ -34,6 +34,7 @@
 #include "mf.cuh"
 #include "mf64.cuh"
 #include "coarse.cuh"
+#include "gj.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -1386,6 +1387,7 @@ __global__ void __launch_bounds__(1024) gj_invert_kernel(int n, double *__restri
     }
     __syncthreads();
     const int p = p_s;
+    if (p >= n) continue; // no comparable entry in the column (block-uniform; the flag is set)
     if (p != k)
       for (int j = t; j < n; j += nt)
       {
@@ -1418,7 +1420,7 @@ __global__ void __launch_bounds__(1024) gj_invert_kernel(int n, double *__restri
   for (int k = n - 1; k >= 0; k--)
   {
     int p = piv[k];
-    if (p != k)
+    if (p != k && p < n)
       for (int i = t; i < n; i += nt)
       {
         double tmp = A[(size_t)i * n + k];
@@ -1444,8 +1446,15 @@ int refresh_coarse_inverse(cdgpu_ctx *ctx, Hierarchy &h)
     if ((rc = dev_alloc(ctx, &h.d_cinv, (size_t)na * na)) || (rc = dev_alloc(ctx, &h.d_cpiv, na + 1)))
       return rc;
   }
-  CD_CUDA(ctx, cudaMemsetAsync(h.d_cpiv + na, 0, sizeof(int), ctx->stream));
-  if (na > 0)
+  if (na > 0 && na <= kGjWarpRows)
+  {
+    (void)cd_launch(gj_warp_kernel, 1, 32, 0, ctx->stream, na, s.d_row_ptr, s.d_dir_start, s.d_kcol, s.d_a, h.d_cinv,
+                    h.d_cpiv + na);
+    CD_LAUNCHED(ctx);
+  }
+  else
+    CD_CUDA(ctx, cudaMemsetAsync(h.d_cpiv + na, 0, sizeof(int), ctx->stream));
+  if (na > kGjWarpRows)
   {
     (void)cd_launch(csr_to_dense_kernel, na, 128, 0, ctx->stream, na, s.d_row_ptr, s.d_kcol, s.d_a, h.d_cinv);
     CD_LAUNCHED(ctx);
