@@ -120,6 +120,7 @@ struct Batch
   int *d_tab = nullptr;
   size_t tab_cap = 0;
   bool dirty = true, check_pending = false;
+  bool tcd_seen = false; // a time-dependent instance has been submitted
   std::vector<int> done_queue;
   size_t bytes = 0;
   // tables of the current running set
@@ -1996,7 +1997,12 @@ int cdgpu_batch_tcd_step(cdgpu_ctx *ctx, int batch_id, int iterations, int *max_
     b.check_pending = false;
   }
   if (b.dirty && (rc = build_tables(ctx, b))) return rc;
-  if (b.tcd_items.K == 0) return fail(ctx, CDGPU_ERR_INVALID, "batch_tcd_step: no time-dependent instance");
+  if (b.tcd_items.K == 0)
+  {
+    if (!b.tcd_seen) return fail(ctx, CDGPU_ERR_INVALID, "batch_tcd_step: no time-dependent instance");
+    if (max_iterations) *max_iterations = 0; // all released
+    return CDGPU_OK;
+  }
   for (auto &in : b.inst)
     if (in.used && in.tcd) in.state = ST_RUN;
   // the step -- right-hand sides, restart of every time-dependent solve from its previous
@@ -2169,7 +2175,9 @@ int cdgpu_batch_release(cdgpu_ctx *ctx, int batch_id, int slot)
     return fail(ctx, CDGPU_ERR_INVALID, "batch_release: bad slot");
   cudaSetDevice(ctx->device);
   BInst &in = b->inst[slot];
-  const bool was_running = in.state == ST_RUN;
+  // a time-dependent instance is in the tables between its steps too, and the row kernels load an
+  // item's matrix entries before they look at its state: the tables are built without it
+  const bool in_tables = in.state == ST_RUN || in.tcd;
   // a running instance leaves the launches first: mark it done on the device
   int st = ST_EMPTY;
   CD_CUDA(ctx, cudaMemcpyAsync(&b->d_ctl[slot].state, &st, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
@@ -2179,7 +2187,7 @@ int cdgpu_batch_release(cdgpu_ctx *ctx, int batch_id, int slot)
   CD_CUDA(ctx, cudaStreamSynchronize(ctx->stream)); // st is a host temporary
   auto &q = b->done_queue;
   q.erase(std::remove(q.begin(), q.end(), slot), q.end());
-  if (was_running) b->dirty = true;
+  if (in_tables) b->dirty = true;
   return CDGPU_OK;
 }
 
@@ -2408,6 +2416,7 @@ static int submit_impl(cdgpu_ctx *ctx, Batch &b, int mg_id, const cdgpu_coeffs *
   b.check_pending = true;
   in.state = tcd ? ST_DONE : ST_RUN;
   in.tcd = tcd != nullptr;
+  b.tcd_seen = b.tcd_seen || in.tcd;
   b.bytes += in.bytes;
   b.dirty = true;
   *slot = sl;
