@@ -188,6 +188,14 @@ int cdgpu_upload_space(cdgpu_ctx *ctx, int dim, int order, int n_cells, const do
     }
   for (int c = 0; c < n_cells && s->all_affine; c++)
     s->all_affine = cell_is_affine(dim, &s->h_coords[(size_t)c * s->nv * dim]);
+  for (int c = 0; c < n_cells; c++)
+    for (int d = 0; d < dim; d++)
+    {
+      const double *v = &s->h_coords[(size_t)c * s->nv * dim + d];
+      double lo = v[0], hi = v[0];
+      for (int k = 1; k < s->nv; k++) lo = std::min(lo, v[k * dim]), hi = std::max(hi, v[k * dim]);
+      s->h_max = std::max(s->h_max, hi - lo);
+    }
   int rc;
   // GlobalNumbers get 4 spare ints: bulk copies of a tile's numbers round their size up to 16 bytes
   if ((rc = dev_alloc(ctx, &s->d_coords, s->h_coords.size())) || (rc = dev_alloc(ctx, &s->d_gn, s->h_gn.size() + 4)))

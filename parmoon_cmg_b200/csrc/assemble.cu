@@ -1028,6 +1028,10 @@ int assemble_space(cdgpu_ctx *ctx, Space &s, int disctype, const double *h_dir, 
   int T = n_tensors(s.dim, disctype), Tr = n_rhs_tensors(s.dim, disctype);
   // the matrix-free operator follows the cell coefficients of an affine assembly only
   s.mf_T = fast ? T : 0;
+  s.cell_peclet = s.co.kind == CDGPU_COEFF_CONSTANT && disctype == CDGPU_GALERKIN
+                      ? std::sqrt(s.co.b1 * s.co.b1 + s.co.b2 * s.co.b2 + (s.dim == 3 ? s.co.b3 * s.co.b3 : 0.0)) *
+                            s.h_max / s.co.eps
+                      : 0.0;
   Coef co = to_coef(s.co);
   if (fast)
   {

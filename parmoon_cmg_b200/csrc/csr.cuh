@@ -239,12 +239,17 @@ __global__ void __launch_bounds__(256, MINB) csr_pipe_kernel(CsrArgs<T> p)
 // Rows of 33-128 entries (8 threads each, 16 loads in flight) keep 4 blocks: 5 and 6 were slower.
 template <typename T> constexpr int csr_blocks(int gs) { return gs == 8 ? 4 : sizeof(T) == 8 ? 5 : 8; }
 
-// grid of a CSR launch: one pass over the rows, at most the resident blocks
-template <typename T> inline int csr_grid(const cdgpu_ctx *ctx, const CsrShape &sh, int rows)
+// grid of a CSR launch: one pass over the rows, at most per_sm blocks per SM
+inline int csr_grid(const cdgpu_ctx *ctx, const CsrShape &sh, int rows, int per_sm)
 {
   const long per_block = 256 / sh.gs;
   const long need = (rows + per_block - 1) / per_block;
-  return (int)std::max<long>(1, std::min<long>(need, (long)ctx->sm_count * csr_blocks<T>(sh.gs)));
+  return (int)std::max<long>(1, std::min<long>(need, (long)ctx->sm_count * per_sm));
+}
+// at most the resident blocks
+template <typename T> inline int csr_grid(const cdgpu_ctx *ctx, const CsrShape &sh, int rows)
+{
+  return csr_grid(ctx, sh, rows, csr_blocks<T>(sh.gs));
 }
 
 template <typename T, int MODE>

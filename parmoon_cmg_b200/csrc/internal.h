@@ -58,6 +58,8 @@ struct Space
   std::vector<double> h_coords;
   std::vector<int> h_gn;
   bool all_affine = true;
+  double h_max = 0;      // longest side of a cell's bounding box
+  double cell_peclet = 0; // |b| h_max / eps of the last assembly, Galerkin with constant coefficients (else 0)
   double *d_coords = nullptr;
   int *d_gn = nullptr;
   // CSR pattern (bit-identical to TSquareStructure + Sort)
@@ -164,6 +166,7 @@ struct Hierarchy
   // the solve's cycles use it from (-1: none), and what the matrix was formed from: the assembly
   // of every level below and the cycle's parameters
   int dense_level = -1, dense_built = -1;
+  int dense_captured[2] = {-1, -1}; // dense_level of the captured cycles
   double *d_dense = nullptr;
   size_t dense_cap = 0;
   std::vector<long> dense_versions;
@@ -181,6 +184,8 @@ struct Hierarchy
   // the running solve applies the finest operator matrix-free in FP64 (Q2 hexahedra from the
   // affine constant-coefficient assembly), not from the CSR entries
   bool mf64 = false;
+  // the running solve's result depends on rounding: its sums keep one order (sums_keep_order)
+  bool keep_order = false;
   cdgpu_solver_params gparams[2] = {};
   long long graph_nodes[2] = {0, 0};
   double **d_io = nullptr;
@@ -341,8 +346,9 @@ int spmv64(cdgpu_ctx *ctx, const Space &s, const double *x, double *y);
 int defect64(cdgpu_ctx *ctx, const Space &s, const double *x, const double *f, double *d,
              double *res);
 int setup_hierarchy_buffers(cdgpu_ctx *ctx, Hierarchy &h, int m);
+// (step: the solve of a time step)
 int run_solve(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, const double *d_rhs,
-              double *d_sol, cdgpu_solve_info *info);
+              double *d_sol, cdgpu_solve_info *info, bool step = false);
 int apply_fp32_form(cdgpu_ctx *ctx, Space &s, int form, const float *d_x, float *d_y);
 int apply_fp64_form(cdgpu_ctx *ctx, Space &s, int form, const double *d_x, double *d_y, bool check);
 // the explicit inverse of the coarsest level's matrix for the exact coarse solve, when its

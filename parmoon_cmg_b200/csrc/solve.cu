@@ -498,16 +498,19 @@ __global__ void __launch_bounds__(kBlock, K <= 24 ? 2 : 1) mf64_row_dots_kernel(
 }
 
 // blocks of a Gram-Schmidt kernel: two per SM (one where K basis values and sums leave registers
-// for one only), never more than the rows need
-static int gs_grid(const cdgpu_ctx *ctx, int n, int k)
+// for one only), never more than the rows need; with keep_order a block per 256 rows, at most four
+// per SM, for every K, so that the sums do not depend on K's row count per thread
+static int gs_grid(const cdgpu_ctx *ctx, const Hierarchy &h, int n, int k)
 {
+  if (h.keep_order) return std::max(1, std::min((n + kBlock - 1) / kBlock, h.gs_stride));
   const int rows = kBlock * (k >= kGsRowsInFlight ? 1 : k >= 8 ? 2 : 4);
   return std::max(1, std::min((n + rows - 1) / rows, ctx->sm_count * (k <= 24 ? 2 : 1)));
 }
 
 // blocks of the product's row phase: its gathers want more rows in flight than the plain passes
-static int row_dots_grid(const cdgpu_ctx *ctx, int n)
+static int row_dots_grid(const cdgpu_ctx *ctx, const Hierarchy &h, int n)
 {
+  if (h.keep_order) return gs_grid(ctx, h, n, 1);
   return std::max(1, std::min((n + kBlock - 1) / kBlock, ctx->sm_count * 2));
 }
 
@@ -1482,7 +1485,7 @@ int refresh_coarse_inverse(cdgpu_ctx *ctx, Hierarchy &h)
 static int choose_dense_level(const Hierarchy &h, const cdgpu_solver_params &p)
 {
   const int L = (int)h.lev.size();
-  if (p.cycle != 1 || p.coarse_smoother != 17 || p.pre < 0 || p.post < 0) return -1;
+  if (h.keep_order || p.cycle != 1 || p.coarse_smoother != 17 || p.pre < 0 || p.post < 0) return -1;
   int best = -1;
   size_t below = 2 * (size_t)h.lev[0].sp->n_active; // shared memory (doubles) of the levels below
   for (int l = 1; l <= L - 2 && l < kVMaxLevels; l++)
@@ -1554,17 +1557,16 @@ int refresh_dense_cycle(cdgpu_ctx *ctx, Hierarchy &h)
   return CDGPU_OK;
 }
 
-// chooses the dense level for a solve, recaptures the cycles when it changed, and forms the matrix
+// chooses the dense level for a solve, recaptures its cycle when it changed, and forms the matrix
 static int prepare_dense_cycle(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p)
 {
-  const int level = choose_dense_level(h, p);
-  if (level != h.dense_level)
-    for (auto &g : h.gexec)
-      if (g)
-      {
-        cudaGraphExecDestroy(g);
-        g = nullptr;
-      }
+  const int level = choose_dense_level(h, p), k = p.precision == 1 ? 1 : 0;
+  if (level != h.dense_captured[k] && h.gexec[k])
+  {
+    cudaGraphExecDestroy(h.gexec[k]);
+    h.gexec[k] = nullptr;
+  }
+  h.dense_captured[k] = level;
   const cdgpu_solver_params &q = h.dense_params;
   if (q.pre != p.pre || q.post != p.post || q.omega != p.omega || q.gmg_damp != p.gmg_damp) h.dense_built = -1;
   h.dense_level = level;
@@ -1609,7 +1611,8 @@ static int finest_defect_norm(cdgpu_ctx *ctx, Hierarchy &h, const double *x, con
     CD_LAUNCHED(ctx);
     return CDGPU_OK;
   }
-  const int grid = defect_grid<double>(ctx, s); // <= 8 blocks per SM, within d_partial
+  // <= 8 blocks per SM, within d_partial (keep_order: that many where the rows need them)
+  const int grid = h.keep_order && s.n_tiles == 0 ? csr_grid(ctx, s.shape, s.n_dof, 8) : defect_grid<double>(ctx, s);
   csr_defect<double>(ctx, s, x, f, d, h.d_partial, grid);
   CD_LAUNCHED(ctx);
   (void)cd_launch(sum_blocks_kernel, 1, 256, 0, ctx->stream, grid, h.d_partial, norm_out_dev);
@@ -1715,7 +1718,7 @@ static int fgmres(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, co
     int rc2;
     // the kernel that formed v_i (scale_norm_kernel or gs_axpy_scale_kernel) set the cycle's slot
     if ((rc2 = precondition(ctx, h, p, V(i), Z(i), true))) return rc2;
-    const int k = i + 1, st = h.gs_stride, grid = gs_grid(ctx, n, k);
+    const int k = i + 1, st = h.gs_stride, grid = gs_grid(ctx, h, n, k);
     double *c = ctl_it(i), *p1 = h.d_partial, *p2 = p1 + (size_t)33 * st;
     int nb1 = grid;
     if (h.mf64 && s.d_inc8)
@@ -1723,7 +1726,7 @@ static int fgmres(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, co
       // w = A z_i matrix-free, its second phase fused with pass 1: h1 = V^T w
       mf64_cells(ctx, s, Z(i));
       CD_LAUNCHED(ctx);
-      nb1 = row_dots_grid(ctx, n);
+      nb1 = row_dots_grid(ctx, h, n);
       launch_row_dots(k, nb1, ctx->stream, n, s.n_active, s.d_inc8, s.d_ybuf64, Z(i), h.d_w, h.d_V, p1, st);
       CD_LAUNCHED(ctx);
     }
@@ -1973,8 +1976,29 @@ static int refresh_mf(cdgpu_ctx *ctx, Hierarchy &h, int precision)
   return CDGPU_OK;
 }
 
+// Whether a mixed solve may end unconverged with sweeps that magnify rounding.  Its result is then
+// whatever the rounding of some 300 FP32 cycles left, and moves with any change of it: the coarse
+// levels as one FP64 product moved such results by up to 9e-5 (2-norm), the Gram-Schmidt sums
+// in another order by up to 8e-6.  So that a call's result stays what it was, these solves keep the
+// FP32 coarse levels and one order of their sums.  (In FP64 the same solves move by 4e-13 at most,
+// and converging ones by rounding.)
+//  * Time steps in 3D: damped Jacobi does not smooth the mass matrix of hexahedra.  The local D^-1 M
+//    of trilinear ones has eigenvalues up to 27/8, so with omega 0.8 a sweep multiplies the upper
+//    modes by -1.7: 32^3 and 48^3 cells end at maxit 300 with ||r|| / ||r0|| of 2e-5 to 0.25.
+//  * Galerkin levels whose convection dominates on their cells: Q2 hexahedra at |b| h / eps of
+//    5 to 12 (8^3 and 12^3 cells, eps 1e-2) end at maxit in half of the cases; at 6 and
+//    below on 16^3 cells they converge in 17-30 iterations, and the benchmark problem has 3.
+constexpr double kPecletKeepOrder = 4.0;
+static bool sums_keep_order(const Hierarchy &h, bool step)
+{
+  if (step) return h.lev.back().sp->dim == 3;
+  for (size_t l = h.lev.size() > 1 ? 1 : 0; l < h.lev.size(); l++)
+    if (h.lev[l].sp->cell_peclet > kPecletKeepOrder) return true;
+  return false;
+}
+
 int run_solve(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, const double *d_rhs, double *d_sol,
-              cdgpu_solve_info *info)
+              cdgpu_solve_info *info, bool step)
 {
   for (auto &L : h.lev)
     if (!L.sp->assembled) return fail(ctx, CDGPU_ERR_INVALID, "solve: every level must be assembled");
@@ -1991,6 +2015,7 @@ int run_solve(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, const 
   // once per pattern, before any capture
   Space &fs = *h.lev.back().sp;
   h.mf64 = solve_mf64(fs);
+  h.keep_order = p.precision == 1 && sums_keep_order(h, step);
   if (p.precision == 0 && (rc = tune_tma(ctx, fs))) return rc;
   if (p.coarse_smoother == 17 && (rc = refresh_coarse_inverse(ctx, h))) return rc;
   if ((rc = prepare_dense_cycle(ctx, h, p))) return rc;

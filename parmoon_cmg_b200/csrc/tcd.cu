@@ -69,6 +69,7 @@ struct TcdLevel
 struct TcdArgs
 {
   int levels, fine; // fine: lev[0] is the finest level
+  int in_order;     // the right-hand side's sums over a row's entries one after the other
   double c_half, c_restore, c3, c4;
   const double *f_old, *f, *x;
   double *B;
@@ -86,6 +87,15 @@ __global__ void __launch_bounds__(256) tcd_system_kernel(const __grid_constant__
   const bool valid = r < l.n, active = r < l.n_active, rhs = p.fine && k == 0 && active;
   const int j1 = valid ? l.rp[r + 1] : 0;
   double s = 0;
+  const bool in_order = rhs && p.in_order;
+  if (in_order) // every lane the whole row, before any entry of M is replaced
+    for (int j = l.rp[r]; j < j1; j++)
+    {
+      double v = l.M[j];
+      if (l.half) v += p.c_half * l.A[j];
+      s += v * p.x[l.kc[j]];
+    }
+  __syncwarp();
   for (int j0 = valid ? l.rp[r] + lane : 0; j0 < j1; j0 += 8 * U)
   {
     double m[U], a[U], x[U];
@@ -111,7 +121,7 @@ __global__ void __launch_bounds__(256) tcd_system_kernel(const __grid_constant__
       if (active)
       {
         if (l.half) v += p.c_half * a[q];
-        if (rhs) s += v * x[q];
+        if (rhs && !in_order) s += v * x[q];
         v += l.c * a[q];
         double back = v;
         back += p.c_restore * a[q];
@@ -123,8 +133,9 @@ __global__ void __launch_bounds__(256) tcd_system_kernel(const __grid_constant__
     }
   }
   if (!p.fine || k != 0) return; // block-uniform
+  if (!p.in_order) // block-uniform
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, 8);
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, 8);
   if (lane != 0 || !valid) return;
   double b = 0.0;
   b += p.c3 * p.f_old[r];
@@ -259,6 +270,7 @@ int cdgpu_tcd_step_device(cdgpu_ctx *ctx, int tcd_id, const cdgpu_solver_params 
     TcdArgs a;
     a.levels = 0;
     a.fine = top == L - 1;
+    a.in_order = fine_only && p->precision == 1; // sums_keep_order
     a.c_half = -tau * theta2;
     a.c_restore = -tau * theta1;
     a.c3 = tau * theta3;
@@ -289,7 +301,7 @@ int cdgpu_tcd_step_device(cdgpu_ctx *ctx, int tcd_id, const cdgpu_solver_params 
     CD_LAUNCHED(ctx);
   }
   cdgpu_solve_info local{};
-  return run_solve(ctx, h, *p, t->d_B, d_sol, info ? info : &local);
+  return run_solve(ctx, h, *p, t->d_B, d_sol, info ? info : &local, true);
 }
 
 int cdgpu_tcd_step(cdgpu_ctx *ctx, int tcd_id, const cdgpu_solver_params *p, double tau, double theta1,
