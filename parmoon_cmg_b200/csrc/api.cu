@@ -369,6 +369,7 @@ int cdgpu_set_coeffs(cdgpu_ctx *ctx, int space_id, const cdgpu_coeffs *co, const
     int rc = dev_alloc(ctx, &s->d_tab, n);
     if (rc) return rc;
     CD_CUDA(ctx, upload(ctx, s->d_tab, h_table, n * sizeof(double)));
+    CD_CUDA(ctx, cudaStreamSynchronize(ctx->stream)); // the caller's table, page-locked or not, is free again
   }
   s->co_set = true;
   return CDGPU_OK;

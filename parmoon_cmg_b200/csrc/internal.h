@@ -310,8 +310,9 @@ template <typename T> int dev_alloc(cdgpu_ctx *ctx, T **p, size_t n)
   return CDGPU_OK;
 }
 
-// Host array to device memory, ordered before everything enqueued on ctx->stream afterwards; the
-// source may be reused on return.  (A plain cudaMemcpy from pageable memory runs on the legacy
+// Host array to device memory, ordered before everything enqueued on ctx->stream afterwards.  A
+// pageable source, such as the library's own vectors, may be reused on return; a page-locked one is
+// read while the copy runs, so after a caller's array the stream is waited for.  (A plain cudaMemcpy from pageable memory runs on the legacy
 // stream, with which the context's non-blocking streams do not synchronise, and may return while
 // the last staged piece is still on its way; cudaMemset does not wait at all.)
 inline cudaError_t upload(const cdgpu_ctx *ctx, void *dst, const void *src, size_t bytes)
