@@ -138,7 +138,7 @@ int cdgpu_get_pattern(cdgpu_ctx *ctx, int space_id, int *h_row_ptr, int *h_kcol)
  * Replaces the CoeffFct2D/CoeffFct3D callback (include/General/Constants.h:120-125)
  * bound by TDiscreteForm2D/3D.  h_table (kind CDGPU_COEFF_TABLE only):
  * n_cells x n_quad x 6 doubles (eps, b1, b2, b3, c, f) at the assembly's
- * quadrature points, see cdgpu_quadrature_points. */
+ * quadrature points, see cdgpu_quadrature_points; copied before the call returns. */
 int cdgpu_set_coeffs(cdgpu_ctx *ctx, int space_id, const cdgpu_coeffs *coeffs,
                      const double *h_table);
 /* quadrature points (physical coordinates, n_cells x n_quad x dim) at which a
@@ -206,7 +206,8 @@ int cdgpu_defect(cdgpu_ctx *ctx, int space_id, const double *h_x, const double *
 int cdgpu_spmv_device(cdgpu_ctx *ctx, int space_id, const double *d_x, double *d_y);
 /* The FP64 product, defect and Jacobi sweep of a matrix larger than L2 stream its tiles into
  * shared memory with bulk copies; the tile shape (nonzeros per tile, pipeline stages, CTAs
- * per SM) is chosen by timing every variant on the matrix at its first FP64 solve.
+ * per SM) is chosen by timing every variant on the matrix at the first solve that streams it,
+ * or the first FP64 solve.
  * This copies a one-line report of that choice (or "not tuned yet") into buf.  No reference
  * counterpart (MatVect / Defect, src/FE/Blas2.C:11-99, are the operations). */
 int cdgpu_product_tuning(cdgpu_ctx *ctx, int space_id, char *buf, int len);
