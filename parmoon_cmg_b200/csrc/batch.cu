@@ -77,7 +77,7 @@ struct BCtl
   const int *rp, *kc;
   const double *a64;
   double cs[kMaxM], sn[kMaxM], s[kMaxM + 1], y[kMaxM];
-  double dots1[kSlots], dots2[kSlots], nrm2;
+  double dots1[kSlots], dots2[kSlots];
   // time-dependent instances: K = M - tau theta2 A (finest), f = (f, phi), c3/c4 = tau theta3/4
   int tcd, na;
   double c3, c4;
@@ -969,12 +969,16 @@ __device__ void d_solve_y(BCtl &c, int k)
 }
 
 // Hessenberg column j, rotations, residual, stopping tests (FgmresIte.C:410-530); one block per
-// instance, which first adds up h2 = V^T w and ||w - V h2||^2 = ||w||^2 - ||h2||^2 (V orthonormal)
+// instance, which first adds up h2 = V^T w and forms ||w - V h2||.  Where h2 is small against w, as
+// after a first orthogonalisation it is, ||w - V h2||^2 = ||w||^2 - ||h2||^2 (V orthonormal); with
+// ||h2||^2 <= ||w||^2 / 16 the difference loses less than a tenth of a digit.  Where it is not (the
+// Krylov space is exhausted, V no longer orthogonal) the difference cancels and may round to zero, and
+// the block sums the entries' squares itself.
 __global__ void __launch_bounds__(kNT) b_givens(BTab t, BCtl *__restrict__ ctl, const double *__restrict__ partial,
                                                 int maxit, int minit, double div_factor)
 {
   CD_PDL_ENTRY();
-  __shared__ double d2[kSlots], h[kSlots + 1], cs[kMaxM], sn[kMaxM];
+  __shared__ double d2[kSlots], h[kSlots + 1], cs[kMaxM], sn[kMaxM], red[kNT / 32];
   for (int k = blockIdx.x; k < t.K; k += gridDim.x)
   {
     BCtl &c = ctl[t.item[k]];
@@ -994,11 +998,26 @@ __global__ void __launch_bounds__(kNT) b_givens(BTab t, BCtl *__restrict__ ctl, 
       }
     }
     __syncthreads();
+    double n2 = d2[j + 1]; // ||w||^2
+    for (int q = 0; q <= j; q++) n2 -= d2[q] * d2[q];
+    if (!(n2 >= 0.9375 * d2[j + 1])) // the same in every thread
+    {
+      double sq = 0;
+      for (int r = threadIdx.x; r < c.n; r += kNT)
+      {
+        double v = c.w[r];
+        for (int q = 0; q <= j; q++) v -= d2[q] * c.V[(size_t)q * c.n + r];
+        sq += v * v;
+      }
+      sq = bsum<32>(sq);
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sq;
+      __syncthreads();
+      n2 = 0;
+      for (int g = 0; g < kNT / 32; g++) n2 += red[g];
+    }
     if (threadIdx.x == 0)
     {
-      double n2 = d2[j + 1];
-      for (int q = 0; q <= j; q++) n2 -= d2[q] * d2[q];
-      const double hn = sqrt(n2 > 0.0 ? n2 : 0.0);
+      const double hn = sqrt(n2);
       h[j + 1] = hn;
       c.hn = hn;
       for (int q = 0; q < j; q++) d_app_rot(h[q], h[q + 1], cs[q], sn[q]);
