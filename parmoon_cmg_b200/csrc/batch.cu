@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(kNT) b_jacobi_first(BTab t, const BCtl *__rest
 //   BR_COLOR     one colour class of an SOR sweep, in place on v[0]
 //   BR_DEFECT    def = f - A v[src]
 //   BR_RESTRICT  coarse f = R def on active coarse rows (zero elsewhere); coarse v[0] = 0, or with
-//                omega the first Jacobi sweep from zero, coarse v[1] = omega D^{-1} f
+//                dst 1 the first Jacobi sweep from zero, coarse v[1] = omega D^{-1} f
 //   BR_PROLONG   v[dst] += omega P (coarse v[src]) on active rows
 // A block takes a contiguous range of virtual blocks, so it looks an instance up once and then
 // walks its rows, the next rows' pointers and entries loaded while the present ones are summed;
@@ -392,10 +392,10 @@ template <int OP> __global__ void __launch_bounds__(kNT, kRowBlocks) b_rows(cons
     const int na = OP == BR_RESTRICT ? L.nca : OP == BR_JACOBI ? L.na : n; // rows with a sum
     const int *list = OP == BR_COLOR ? L.color_rows + __ldg(p.cstart + k) : nullptr;
     constexpr bool kSweep = OP == BR_JACOBI || OP == BR_COLOR;
-    const bool scale = kSweep || (OP == BR_RESTRICT && p.omega != 0.f); // the result is divided by the diagonal
+    const bool scale = kSweep || (OP == BR_RESTRICT && p.dst == 1); // the result is divided by the diagonal
     const float *dg = OP == BR_RESTRICT ? C.d32 : L.d32, *f = L.rhs;
     float *y = OP == BR_RESTRICT ? C.rhs : OP == BR_DEFECT ? L.def : OP == BR_COLOR ? L.v[0] : L.v[p.dst & 1];
-    float *y0 = OP == BR_RESTRICT ? C.v[p.omega != 0.f ? 1 : 0] : nullptr;
+    float *y0 = OP == BR_RESTRICT ? C.v[p.dst] : nullptr;
     const float *own = OP == BR_JACOBI ? x : y; // the vector an update adds to
     const int updates =
         OP == BR_COLOR && p.sweeps ? ssor_updates(p.color, L.n_colors, p.back, p.sweep, p.sweeps) : 1;
@@ -471,7 +471,7 @@ template <int OP> __global__ void __launch_bounds__(kNT, kRowBlocks) b_rows(cons
         else if (OP == BR_RESTRICT)
         {
           y[row] = row < na ? s : 0.f;
-          y0[row] = p.omega != 0.f && row < na ? p.omega * s / dr : 0.f;
+          y0[row] = p.dst == 1 && row < na ? p.omega * s / dr : 0.f;
         }
         else
           y[row] = o + p.omega * s;
@@ -1682,7 +1682,7 @@ static int batch_cycle(cdgpu_ctx *ctx, Batch &b)
     int rc = sweeps(d, pre, true);
     if (rc) return rc;
     if ((rc = rows(b_rows<BR_DEFECT>, b.smooth[d], d, after_pre, 0, 0.f))) return rc;
-    if ((rc = rows(b_rows<BR_RESTRICT>, b.restrict_[d], d, 0, 0, jac && pre > 0 ? omega : 0.f))) return rc;
+    if ((rc = rows(b_rows<BR_RESTRICT>, b.restrict_[d], d, 0, jac && pre > 0 ? 1 : 0, omega))) return rc;
   }
   if (b.cta_smem > 0)
   {
