@@ -1469,7 +1469,7 @@ static int build_tables(cdgpu_ctx *ctx, Batch &b)
   b.cta_smem = 0;
   for (int i : b.run) b.cta_smem = std::max(b.cta_smem, b.inst[i].cta_smem);
   if (b.cta_smem > 48 * 1024)
-    CD_CUDA(ctx, cudaFuncSetAttribute(b_cta_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.cta_smem));
+    CD_CUDA(ctx, cudaFuncSetAttribute(b_cta_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynShared));
   std::vector<int> pack;
   struct Pending { BTab *t; size_t item_off, bs_off; };
   std::vector<Pending> pend;

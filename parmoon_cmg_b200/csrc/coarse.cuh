@@ -24,7 +24,7 @@
 constexpr int kDenseRows = 1024;
 constexpr int kVMaxLevels = 12;
 constexpr int kVThreads = 1024;
-constexpr size_t kVSharedBytes = 220 * 1024; // vectors of a CTA's columns
+constexpr size_t kVSharedBytes = 220 * 1024; // of a CTA, at most (vcycle_layout); below kMaxDynShared
 
 struct VLevel
 {

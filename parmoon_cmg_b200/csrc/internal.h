@@ -310,6 +310,11 @@ template <typename T> int dev_alloc(cdgpu_ctx *ctx, T **p, size_t n)
   return CDGPU_OK;
 }
 
+// Most dynamic shared memory a block of a kernel without static shared memory may ask for.  The limit
+// of a function belongs to the process: set to the size of one problem, it would be lowered under
+// another context's or batch's launches and captures, so it is only ever set to this.
+constexpr int kMaxDynShared = 227 * 1024;
+
 // Host array to device memory, ordered before everything enqueued on ctx->stream afterwards.  A
 // pageable source, such as the library's own vectors, may be reused on return; a page-locked one is
 // read while the copy runs, so after a caller's array the stream is waited for.  (A plain cudaMemcpy from pageable memory runs on the legacy

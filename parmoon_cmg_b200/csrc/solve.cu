@@ -1487,12 +1487,13 @@ static int choose_dense_level(const Hierarchy &h, const cdgpu_solver_params &p)
   const int L = (int)h.lev.size();
   if (h.keep_order || p.cycle != 1 || p.coarse_smoother != 17 || p.pre < 0 || p.post < 0) return -1;
   int best = -1;
-  size_t below = 2 * (size_t)h.lev[0].sp->n_active; // shared memory (doubles) of the levels below
+  VCycleArgs v;
+  v.lev[0].na = h.lev[0].sp->n_active;
   for (int l = 1; l <= L - 2 && l < kVMaxLevels; l++)
   {
-    const size_t na = h.lev[l].sp->n_active;
-    if (na > (size_t)kDenseRows || (below + 3 * na) * sizeof(double) > kVSharedBytes) break;
-    below += 4 * na;
+    v.top = l;
+    v.lev[l].na = h.lev[l].sp->n_active;
+    if (v.lev[l].na > kDenseRows || vcycle_layout(v, 1) > kVSharedBytes) break;
     best = l;
   }
   return best;
@@ -1549,7 +1550,7 @@ int refresh_dense_cycle(cdgpu_ctx *ctx, Hierarchy &h)
   auto kern = C == 1 ? vcycle_matrix_kernel<1> : C == 2 ? vcycle_matrix_kernel<2> : C == 4 ? vcycle_matrix_kernel<4>
                                                                                            : vcycle_matrix_kernel<8>;
   const size_t sm = vcycle_layout(v, C);
-  CD_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  CD_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynShared));
   (void)cd_launch(kern, std::max(1, (na + C - 1) / C), kVThreads, sm, ctx->stream, v);
   CD_LAUNCHED(ctx);
   h.dense_built = top;
