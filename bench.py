@@ -174,6 +174,10 @@ def cpu_count():
 def run_reference_arm(args, rank, world):
     if rank != 0:
         return
+    if not os.path.exists(os.path.join(ROOT, "oracle", "_ref", "cd3d_dump")):
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/cd3d_dump is not built here "
+                          "(oracle/build_ref.py compiles it from the reference's sources)"}), flush=True)
+        return
     cores = cpu_count()
     # one reference process per core, each solving the workload; memory bound ~1.5 GB each
     try:
