@@ -907,7 +907,9 @@ __device__ __forceinline__ void b_gs_rows(const BCtl &c, int kk, const double *h
 }
 
 // AXPY false: partial sums of h1 = V^T w in p2; true: h1 from p1 (kept in ctl.dots1), w -= V h1,
-// partial sums of h2 = V^T w and ||w||^2 in p2
+// partial sums of h2 = V^T w and ||w||^2 in p2.  (With 25 to 32 vectors the basis values, their sums
+// and the row do not fit the 128 registers of two blocks per SM: 344 bytes of spill stores and 176 of
+// loads a thread in the AXPY form.)
 template <bool AXPY>
 __global__ void __launch_bounds__(kNT, 2) b_gs(BTab t, BCtl *__restrict__ ctl, const double *__restrict__ p1,
                                                double *__restrict__ p2)

@@ -12,7 +12,8 @@
 // (7.4 MB) is read from L2 by all SMs at once, its first entries before the predecessor of the
 // product has finished.  Measured per solve, the launched levels against the dense product
 // (formation included): CD2D Q1 64^2 (28 launches of each FGMRES iteration saved) 1415 -> 959 us,
-// CD2D Q2 192^2 4280 -> 3810, CD3D Q2 32^3 mixed 3734 -> 3630.
+// CD2D Q2 192^2 4280 -> 3810, CD3D Q2 32^3 mixed 3734 -> 3630.  Mixed solves that may end
+// unconverged keep the launched FP32 levels (sums_keep_order in solve.cu).
 #pragma once
 
 #include "internal.h"
@@ -188,7 +189,8 @@ template <int C, int MODE> __device__ __forceinline__ void v_pass(const VPass &p
 }
 
 // One CTA forms C columns of B, its vectors in shared memory, column-major.  Dirichlet rows and
-// columns carry zeros throughout a coarse cycle and are skipped.
+// columns carry zeros throughout a coarse cycle and are skipped.  (8 columns at 1,024 threads leave 64
+// registers a thread: 52 bytes of spill stores, 128 of loads.)
 template <int C>
 __global__ void __launch_bounds__(kVThreads, 1) vcycle_matrix_kernel(const __grid_constant__ VCycleArgs v)
 {

@@ -262,12 +262,13 @@ int cuda_fail(cdgpu_ctx *ctx, cudaError_t e, const char *what);
 // (griddepcontrol.wait) before it reads or writes anything the predecessor may touch, and
 // only then lets its own successor be scheduled (griddepcontrol.launch_dependents).  So at
 // most two kernels of a chain are resident at once, and the later one runs only the part
-// before its wait (the batch's row passes, many short launches in a row, let their successor in
-// at once: several may be resident, each still waiting for all before it, and what they read
-// before the wait is written by no kernel of the cycle): the launch, the CTA scheduling and, in kernels of the captured multigrid
+// before its wait: the launch, the CTA scheduling and, in kernels of the captured multigrid
 // cycle, loads of data that no kernel of the cycle writes (matrices, transfer operators,
 // incidence lists, reference tensors).  Without the launch attribute both instructions
 // return at once.
+// The batch's row passes (b_rows), many short launches in a row, let their successor in before
+// their own wait.  Several of them may then be resident, each still waiting for all before it, and
+// what they read before the wait is written by no kernel of the cycle.
 #define CD_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
 #define CD_PDL_TRIGGER() asm volatile("griddepcontrol.launch_dependents;" ::: "memory")
 #define CD_PDL_ENTRY() \
@@ -352,6 +353,8 @@ int spmv64(cdgpu_ctx *ctx, const Space &s, const double *x, double *y);
 int defect64(cdgpu_ctx *ctx, const Space &s, const double *x, const double *f, double *d,
              double *res);
 int setup_hierarchy_buffers(cdgpu_ctx *ctx, Hierarchy &h, int m);
+// whether a time step's sums keep one order (sums_keep_order in solve.cu)
+bool step_keeps_order(const Space &finest, int precision);
 // (step: the solve of a time step)
 int run_solve(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, const double *d_rhs,
               double *d_sol, cdgpu_solve_info *info, bool step = false);

@@ -330,6 +330,7 @@ __global__ void __launch_bounds__(QuadLane<DIM, P, FORM>::THREADS) quad_lane_ker
 // ---------------------------------------------------------------------------
 // Q2 hexahedra
 // ---------------------------------------------------------------------------
+// (two blocks per SM leave 128 registers: 32-40 bytes of spill stores, 36-52 of loads, by form)
 constexpr int kQ27Cells = 5, kQ27Threads = 256;
 
 // products of one-dimensional functions at the points: [q][i * 3 + j], i the test function

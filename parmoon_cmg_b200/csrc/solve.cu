@@ -261,9 +261,9 @@ __global__ void coarse_smooth_kernel(int n, int n_active, const int *__restrict_
 // shuffles.  The minimum of two blocks per SM in the launch bounds is there for the compiler's
 // scheduling: without it the axpy-scale kernel was built with 32 registers, a few loads in
 // flight, and took 12.8 us instead of 8.7.
-constexpr int kGsRowsInFlight = 16; // basis values a thread keeps in flight: rows per thread = 16 / K
+constexpr int kGsRowsInFlight = 16; // from this K on a thread has enough basis values in flight with one row
 
-// rows a thread takes at once, so that small K keeps as many loads in flight as large K
+// rows a thread takes at once, so that small K keeps loads in flight too
 template <int K> constexpr int gs_rows() { return K >= kGsRowsInFlight ? 1 : K >= 8 ? 2 : 4; }
 
 // a block's sums of acc[0..N) (and, with NORM, of sq in slot N) into partial[slot * stride +
@@ -1481,7 +1481,8 @@ int refresh_coarse_inverse(cdgpu_ctx *ctx, Hierarchy &h)
 
 // The level whose V-cycle a solve with parameters p applies as a dense matrix, or -1.  V-cycles
 // with the exact coarse solve only (the other coarse smoothers iterate until a residual drops and
-// are not linear); below the finest level, whose right-hand side has Dirichlet entries.
+// are not linear); below the finest level, whose right-hand side has Dirichlet entries; not where the
+// result depends on the rounding of FP32 coarse levels (sums_keep_order).
 static int choose_dense_level(const Hierarchy &h, const cdgpu_solver_params &p)
 {
   const int L = (int)h.lev.size();
@@ -1983,18 +1984,27 @@ static int refresh_mf(cdgpu_ctx *ctx, Hierarchy &h, int precision)
 // in another order by up to 8e-6.  So that a call's result stays what it was, these solves keep the
 // FP32 coarse levels and one order of their sums.  (In FP64 the same solves move by 4e-13 at most,
 // and converging ones by rounding.)
-//  * Time steps in 3D: damped Jacobi does not smooth the mass matrix of hexahedra.  The local D^-1 M
-//    of trilinear ones has eigenvalues up to 27/8, so with omega 0.8 a sweep multiplies the upper
-//    modes by -1.7: 32^3 and 48^3 cells end at maxit 300 with ||r|| / ||r0|| of 2e-5 to 0.25.
-//  * Galerkin levels whose convection dominates on their cells: Q2 hexahedra at |b| h / eps of
-//    5 to 12 (8^3 and 12^3 cells, eps 1e-2) end at maxit in half of the cases; at 6 and
-//    below on 16^3 cells they converge in 17-30 iterations, and the benchmark problem has 3.
-constexpr double kPecletKeepOrder = 4.0;
-static bool sums_keep_order(const Hierarchy &h, bool step)
+//  * Time steps on more than 16^3 hexahedra: damped Jacobi does not smooth their mass matrix.  The
+//    local D^-1 M of trilinear ones has eigenvalues up to 27/8, so with omega 0.8 a sweep multiplies the
+//    upper modes by -1.7: steps of 1e-6 to 1e-1 on 16^3 cells converge in 9-61 iterations, on 20^3
+//    and 24^3 they may not, from 32^3 on (1e-2 and below) they end at maxit 300 with ||r|| / ||r0|| of 2e-5 to 0.25.
+//  * Galerkin levels whose convection dominates on their cells.  With |b| h / eps of 8 and above
+//    triquadratic solves end at maxit (8^3 to 32^3 cells), biquadratic ones from 6.5 on (32^2, 128^2); at 6
+//    they take 20-78 iterations, and the benchmark problem has 3.  Bilinear ones end there from 1.5 on
+//    (128^2; 4 on 32^2), trilinear ones from 2.5 on (48^3; 5 on 16^3), at 1 they take 7-30.
+// Kept so, 300 iterations take 14.6 -> 19.7 ms (step, 32^3 cells), 24.8 -> 30.5 (48^3) and 11.7 -> 14.7 ms
+// (Galerkin Q2, 8^3).
+constexpr int kStepKeepCells = 4096;
+bool step_keeps_order(const Space &finest, int precision)
 {
-  if (step) return h.lev.back().sp->dim == 3;
+  return precision == 1 && finest.dim == 3 && finest.n_cells > kStepKeepCells;
+}
+static bool sums_keep_order(const Hierarchy &h, int precision, bool step)
+{
+  if (step) return step_keeps_order(*h.lev.back().sp, precision);
+  if (precision != 1) return false;
   for (size_t l = h.lev.size() > 1 ? 1 : 0; l < h.lev.size(); l++)
-    if (h.lev[l].sp->cell_peclet > kPecletKeepOrder) return true;
+    if (h.lev[l].sp->cell_peclet > (h.lev[l].sp->order == 1 ? 1.0 : 6.0)) return true;
   return false;
 }
 
@@ -2018,7 +2028,7 @@ int run_solve(cdgpu_ctx *ctx, Hierarchy &h, const cdgpu_solver_params &p, const 
   // form tunes beside the matrix-free operator too, for the products its callers ask for.
   Space &fs = *h.lev.back().sp;
   h.mf64 = solve_mf64(fs);
-  h.keep_order = p.precision == 1 && sums_keep_order(h, step);
+  h.keep_order = sums_keep_order(h, p.precision, step);
   if ((!h.mf64 || p.precision == 0) && (rc = tune_tma(ctx, fs))) return rc;
   if (p.coarse_smoother == 17 && (rc = refresh_coarse_inverse(ctx, h))) return rc;
   if ((rc = prepare_dense_cycle(ctx, h, p))) return rc;

@@ -270,7 +270,7 @@ int cdgpu_tcd_step_device(cdgpu_ctx *ctx, int tcd_id, const cdgpu_solver_params 
     TcdArgs a;
     a.levels = 0;
     a.fine = top == L - 1;
-    a.in_order = fine_only && p->precision == 1; // sums_keep_order
+    a.in_order = step_keeps_order(f, p->precision);
     a.c_half = -tau * theta2;
     a.c_restore = -tau * theta1;
     a.c3 = tau * theta3;
